@@ -5,7 +5,6 @@
 // value plus the four fine face values, computed by the coarse block's CTA
 // from the fine blocks' face cells and their ghosts.
 #include <algorithm>
-#include <type_traits>
 
 #include "../../include/cup3d_b200.h"
 #include "lab.cuh"
@@ -19,57 +18,6 @@ struct Vec3 {
   double v[3];
 };
 
-// ---------------------------------------------------------------------------
-// AdvectionDiffusion: KernelAdvectDiffuse (AdvectionDiffusion.cpp:19-215)
-// ---------------------------------------------------------------------------
-__device__ __forceinline__ double sq(double a) { return a * a; }
-
-// WENO5 reconstruction biased to the left (weno5_plus of
-// AdvectionDiffusion.cpp:34-64): candidate stencils f1..f3 with smoothness
-// indicators b1..b3, nonlinear weights w_k = (d_k/q_k) / sum_j d_j/q_j with
-// q_k = (b_k + eps)^2 and d = (0.1, 0.6, 0.3).  The weights are evaluated with
-// one division instead of four: multiplying numerator and denominator by
-// q1 q2 q3 gives  sum_k a_k f_k / sum_k a_k  with  a_1 = 0.1 q2 q3,
-// a_2 = 0.6 q1 q3, a_3 = 0.3 q1 q2  (q_k >= eps^2 = 1e-12, so no underflow).
-__device__ __forceinline__ double weno5_left(double um2, double um1, double u, double up1, double up2) {
-  const double e = 1e-6;
-  const double b1 = 13.0 / 12.0 * sq((um2 + u) - 2 * um1) + 0.25 * sq((um2 + 3 * u) - 4 * um1);
-  const double b2 = 13.0 / 12.0 * sq((um1 + up1) - 2 * u) + 0.25 * sq(um1 - up1);
-  const double b3 = 13.0 / 12.0 * sq((u + up2) - 2 * up1) + 0.25 * sq((3 * u + up2) - 4 * up1);
-  const double q1 = sq(b1 + e), q2 = sq(b2 + e), q3 = sq(b3 + e);
-  const double a1 = 0.1 * (q2 * q3), a2 = 0.6 * (q1 * q3), a3 = 0.3 * (q1 * q2);
-  const double f1 = (11.0 / 6.0) * u + ((1.0 / 3.0) * um2 - (7.0 / 6.0) * um1);
-  const double f2 = (5.0 / 6.0) * u + ((-1.0 / 6.0) * um1 + (1.0 / 3.0) * up1);
-  const double f3 = (1.0 / 3.0) * u + ((+5.0 / 6.0) * up1 - (1.0 / 6.0) * up2);
-  return ((a1 * f1 + a3 * f3) + a2 * f2) / ((a1 + a3) + a2);
-}
-
-// Upwind derivative of KernelAdvectDiffuse (AdvectionDiffusion.cpp:66-103).
-// WENO5: the right-biased reconstruction (weno5_minus) is the left-biased one
-// of the mirrored stencil, weno5_minus(a,b,c,d,e) = weno5_plus(e,d,c,b,a), so
-// the upwind choice only selects the five inputs of two left-biased
-// evaluations and no warp diverges on the sign of U.
-template <int SCHEME>
-__device__ __forceinline__ double deriv(double U, double um3, double um2, double um1, double u, double up1,
-                                        double up2, double up3) {
-  if (SCHEME == 1) {
-    const bool pos = U > 0;
-    // face i+1/2 and face i-1/2 reconstructions in the upwind direction
-    const double fp = weno5_left(pos ? um2 : up3, pos ? um1 : up2, pos ? u : up1, pos ? up1 : u, pos ? up2 : um1);
-    const double fm = weno5_left(pos ? um3 : up2, pos ? um2 : up1, pos ? um1 : u, pos ? u : um1, pos ? up1 : um2);
-    return fp - fm;
-  }
-  if (U > 0) return (-2 * um3 + 15 * um2 - 60 * um1 + 20 * u + 30 * up1 - 3 * up2) / 60.;
-  return (2 * up3 - 15 * up2 + 60 * up1 - 20 * u - 30 * um1 + 3 * um2) / 60.;
-}
-
-__device__ __forceinline__ bool has_finer(const DevMesh& M, int b) {
-  bool r = false;
-#pragma unroll
-  for (int f = 0; f < 6; ++f) r |= M.fkind[b * 6 + f] == K_FINER;
-  return r;
-}
-
 // lab coordinates of own face cell (layer 0) and the ghost at layer 1
 __device__ __forceinline__ void face_lab_pair(int d, int s, int a, int bb, int q[3], int g[3]) {
   q[d] = s ? BS - 1 : 0;
@@ -79,233 +27,6 @@ __device__ __forceinline__ void face_lab_pair(int d, int s, int a, int bb, int q
   g[1] = q[1];
   g[2] = q[2];
   g[d] += s ? 1 : -1;
-}
-
-template <int SCHEME>
-__global__ void __launch_bounds__(NT, 3)
-    k_advect_stage(DevMesh M, const double* __restrict__ vin, double* __restrict__ vout, double* tmpV, double dt,
-                   double nu, Vec3 ui, int stage) {
-  extern __shared__ double smem[];
-  using LG = LabGeom<3>;
-  double* lab = smem;
-  double* corr = smem + 3 * LG::V;
-  const size_t n = size_t(M.nb) * BN;
-  const double alpha = stage == 0 ? 1.0 / 3.0 : (stage == 1 ? 15.0 / 16.0 : 8.0 / 15.0);
-  const double beta = stage == 0 ? -5.0 / 9.0 : (stage == 1 ? -153.0 / 128.0 : 0.0);
-  auto get = [&](int c, int blk, int cell) { return vin[c * n + size_t(blk) * BN + cell]; };
-  for (int b = blockIdx.x; b < M.nb; b += gridDim.x) {
-    __syncthreads();
-    lab_fill<3, 3>(lab, M, b, get, true);
-    const bool fix = has_finer(M, b);
-    if (fix)
-      for (int i = threadIdx.x; i < 3 * BN; i += NT) corr[i] = 0.0;
-    __syncthreads();
-    const double h = M.h[b], h3 = h * h * h;
-    const double dtb = block_dt(M, b, dt);
-    const double facA = -dtb / h * h3;
-    const double facD = (nu / h) * (dtb / h) * h3;
-    if (fix) {
-      for (int f = 0; f < 6; ++f) {
-        if (M.fkind[b * 6 + f] != K_FINER) continue;
-        const int d = f >> 1, s = f & 1;
-        if (threadIdx.x < 64) {
-          const int a = threadIdx.x & 7, bb = threadIdx.x >> 3;
-          int q[3], g[3];
-          face_lab_pair(d, s, a, bb, q, g);
-          const int ch = M.fnbr[b * 24 + 4 * f + (a >> 2) + 2 * (bb >> 2)];
-          const double hf = M.h[ch];
-          const double facDf = (nu / hf) * (dtb / hf) * hf * hf * hf;
-          const int oc = face_cell(d, s, 0, a, bb);
-#pragma unroll
-          for (int c = 0; c < 3; ++c) {
-            double val = facD * (lab[c * LG::V + LG::at(q[0], q[1], q[2])] - lab[c * LG::V + LG::at(g[0], g[1], g[2])]);
-#pragma unroll
-            for (int e2 = 0; e2 < 2; ++e2)
-#pragma unroll
-              for (int e1 = 0; e1 < 2; ++e1) {
-                const int fa = 2 * (a & 3) + e1, fb = 2 * (bb & 3) + e2;
-                const double uf = vin[c * n + size_t(ch) * BN + face_cell(d, 1 - s, 0, fa, fb)];
-                const double gf = child_ghost1([&](int cell) { return vin[c * n + size_t(b) * BN + cell]; }, M,
-                                               ch, d, s, fa, fb);
-                val += facDf * (uf - gf);
-              }
-            corr[c * BN + oc] += val;
-          }
-        }
-        __syncthreads();
-      }
-    }
-    if (SCHEME == 1) {
-      // WENO5: each face value is reconstructed once where the cells on both
-      // sides take the same upwind side.  Per direction: every cell
-      // reconstructs its upper face into fbuf; the lower faces of the first
-      // cells of the lines go to fstart; a cell then takes its lower face from
-      // the cell below, or reconstructs it itself where the upwind sign flips.
-      // The face values are those of deriv<1> (the same reconstruction of the
-      // same inputs), so the result does not change.
-      double* fbuf = corr + 3 * BN;   // 3 x 512: upper faces along the current direction
-      double* fstart = fbuf + 3 * BN; // 3 x 64: lower faces of the lines' first cells
-      auto L = [&](int c, int xx, int yy, int zz) { return lab[c * LG::V + LG::at(xx, yy, zz)]; };
-      double der[2][3][3];  // [cell slot][component][direction]
-      auto direction = [&](auto dconst) {
-        constexpr int d = decltype(dconst)::value;
-        constexpr int stride = d == 0 ? 1 : (d == 1 ? 8 : 64);
-        // reconstruction at the upper face of cell (p0, p1, p2) along d with
-        // the upwind side pos, as deriv<1>'s fp
-        auto face_up = [&](int c, int p0, int p1, int p2, bool pos) {
-          auto at = [&](int k) {
-            return L(c, p0 + (d == 0 ? k : 0), p1 + (d == 1 ? k : 0), p2 + (d == 2 ? k : 0));
-          };
-          const double um2 = at(-2), um1 = at(-1), u0 = at(0), up1 = at(1), up2 = at(2), up3 = at(3);
-          return weno5_left(pos ? um2 : up3, pos ? um1 : up2, pos ? u0 : up1, pos ? up1 : u0, pos ? up2 : um1);
-        };
-#pragma unroll 1
-        for (int qq = 0; qq < 2; ++qq) {
-          const int cell = threadIdx.x + qq * NT;
-          const int x = cell & 7, y = (cell >> 3) & 7, z = cell >> 6;
-          const bool pos = L(d, x, y, z) + ui.v[d] > 0;
-#pragma unroll 1
-          for (int c = 0; c < 3; ++c) fbuf[c * BN + cell] = face_up(c, x, y, z, pos);
-        }
-        if (threadIdx.x < 3 * 64) {
-          const int c = threadIdx.x >> 6, line = threadIdx.x & 63;
-          const int t1 = line & 7, t2 = line >> 3;
-          const int x = d == 0 ? 0 : t1, y = d == 1 ? 0 : (d == 0 ? t1 : t2), z = d == 2 ? 0 : t2;
-          const bool pos = L(d, x, y, z) + ui.v[d] > 0;  // the first cell's side
-          fstart[c * 64 + line] = face_up(c, x - (d == 0), y - (d == 1), z - (d == 2), pos);
-        }
-        __syncthreads();
-#pragma unroll
-        for (int qq = 0; qq < 2; ++qq) {
-          const int cell = threadIdx.x + qq * NT;
-          const int x = cell & 7, y = (cell >> 3) & 7, z = cell >> 6;
-          const int pd = d == 0 ? x : (d == 1 ? y : z);
-          const bool pos = L(d, x, y, z) + ui.v[d] > 0;
-          double fm[3];
-          if (pd == 0) {
-            const int line = d == 0 ? y + 8 * z : (d == 1 ? x + 8 * z : x + 8 * y);
-#pragma unroll
-            for (int c = 0; c < 3; ++c) fm[c] = fstart[c * 64 + line];
-          } else {
-            const int xm = x - (d == 0), ym = y - (d == 1), zm = z - (d == 2);
-            const bool pos_m = L(d, xm, ym, zm) + ui.v[d] > 0;
-            if (pos_m == pos) {
-#pragma unroll
-              for (int c = 0; c < 3; ++c) fm[c] = fbuf[c * BN + cell - stride];
-            } else {  // the upwind side flips between the two cells
-#pragma unroll
-              for (int c = 0; c < 3; ++c) fm[c] = face_up(c, xm, ym, zm, pos);
-            }
-          }
-#pragma unroll
-          for (int c = 0; c < 3; ++c) der[qq][c][d] = fbuf[c * BN + cell] - fm[c];
-        }
-        __syncthreads();
-      };
-      direction(std::integral_constant<int, 0>{});
-      direction(std::integral_constant<int, 1>{});
-      direction(std::integral_constant<int, 2>{});
-#pragma unroll 1
-      for (int qq = 0; qq < 2; ++qq) {
-        const int cell = threadIdx.x + qq * NT;
-        const int x = cell & 7, y = (cell >> 3) & 7, z = cell >> 6;
-        const double uA[3] = {L(0, x, y, z) + ui.v[0], L(1, x, y, z) + ui.v[1], L(2, x, y, z) + ui.v[2]};
-        double out[3];
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-          const double dx = der[qq][c][0], dy = der[qq][c][1], dz = der[qq][c][2];
-          const double sx = L(c, x + 1, y, z) + L(c, x - 1, y, z);
-          const double sy = L(c, x, y + 1, z) + L(c, x, y - 1, z);
-          const double sz = L(c, x, y, z + 1) + L(c, x, y, z - 1);
-          double dD, dA;
-          if (c == 0) {
-            dD = (sx + (sy + sz)) - 6 * L(0, x, y, z);
-            dA = uA[0] * dx + (uA[1] * dy + uA[2] * dz);
-          } else if (c == 1) {
-            dD = (sy + (sz + sx)) - 6 * L(1, x, y, z);
-            dA = uA[1] * dy + (uA[2] * dz + uA[0] * dx);
-          } else {
-            dD = (sz + (sx + sy)) - 6 * L(2, x, y, z);
-            dA = uA[2] * dz + (uA[0] * dx + uA[1] * dy);
-          }
-          out[c] = facA * dA + facD * dD;
-        }
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-          const size_t gi = c * n + size_t(b) * BN + cell;
-          double tot = (stage ? tmpV[gi] : 0.0) + out[c];
-          if (fix) tot += corr[c * BN + cell];
-          vout[gi] = L(c, x, y, z) + tot * (alpha / h3);
-          if (stage < 2) tmpV[gi] = tot * beta;
-        }
-      }
-      continue;
-    }
-    // the cell and component loops stay rolled: the unrolled body (18 WENO
-    // reconstructions per cell) overflowed the instruction cache (the top
-    // stall was no_instruction); rolled, a stage takes 188 us instead of 204
-#pragma unroll 1
-    for (int qq = 0; qq < 2; ++qq) {
-      const int cell = threadIdx.x + qq * NT;
-      const int x = cell & 7, y = (cell >> 3) & 7, z = cell >> 6;
-      auto L = [&](int c, int xx, int yy, int zz) { return lab[c * LG::V + LG::at(xx, yy, zz)]; };
-      const double uA[3] = {L(0, x, y, z) + ui.v[0], L(1, x, y, z) + ui.v[1], L(2, x, y, z) + ui.v[2]};
-      double out[3];
-#pragma unroll 1
-      for (int c = 0; c < 3; ++c) {
-        const double dx = deriv<SCHEME>(uA[0], L(c, x - 3, y, z), L(c, x - 2, y, z), L(c, x - 1, y, z), L(c, x, y, z),
-                                        L(c, x + 1, y, z), L(c, x + 2, y, z), L(c, x + 3, y, z));
-        const double dy = deriv<SCHEME>(uA[1], L(c, x, y - 3, z), L(c, x, y - 2, z), L(c, x, y - 1, z), L(c, x, y, z),
-                                        L(c, x, y + 1, z), L(c, x, y + 2, z), L(c, x, y + 3, z));
-        const double dz = deriv<SCHEME>(uA[2], L(c, x, y, z - 3), L(c, x, y, z - 2), L(c, x, y, z - 1), L(c, x, y, z),
-                                        L(c, x, y, z + 1), L(c, x, y, z + 2), L(c, x, y, z + 3));
-        const double sx = L(c, x + 1, y, z) + L(c, x - 1, y, z);
-        const double sy = L(c, x, y + 1, z) + L(c, x, y - 1, z);
-        const double sz = L(c, x, y, z + 1) + L(c, x, y, z - 1);
-        double dD, dA;
-        if (c == 0) {
-          dD = (sx + (sy + sz)) - 6 * L(0, x, y, z);
-          dA = uA[0] * dx + (uA[1] * dy + uA[2] * dz);
-        } else if (c == 1) {
-          dD = (sy + (sz + sx)) - 6 * L(1, x, y, z);
-          dA = uA[1] * dy + (uA[2] * dz + uA[0] * dx);
-        } else {
-          dD = (sz + (sx + sy)) - 6 * L(2, x, y, z);
-          dA = uA[2] * dz + (uA[0] * dx + uA[1] * dy);
-        }
-        out[c] = facA * dA + facD * dD;
-      }
-#pragma unroll
-      for (int c = 0; c < 3; ++c) {
-        const size_t gi = c * n + size_t(b) * BN + cell;
-        double tot = (stage ? tmpV[gi] : 0.0) + out[c];
-        if (fix) tot += corr[c * BN + cell];
-        vout[gi] = L(c, x, y, z) + tot * (alpha / h3);
-        if (stage < 2) tmpV[gi] = tot * beta;
-      }
-    }
-  }
-}
-
-int launch_advect_stage(const DevMesh& M, const double* vin, double* vout, double* tmpV, double dt, double nu,
-                        const double* uinf, int scheme, int stage, int grid, cudaStream_t s) {
-  // lab, flux correction; WENO5 adds the face buffers (3 x 512 + 3 x 64)
-  const size_t smem = (3 * LabGeom<3>::V + 3 * BN + (scheme == 1 ? 3 * BN + 3 * 64 : 0)) * sizeof(double);
-  static unsigned long long attr_set[2] = {0, 0};
-  Vec3 ui{{uinf[0], uinf[1], uinf[2]}};
-  if (scheme == 1) {
-    if (first_on_device(attr_set[1]))
-      CUP_CUDA_TRY(cudaFuncSetAttribute(k_advect_stage<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
-    ProfScope ps("advect_stage_weno5", s);
-    k_advect_stage<1><<<grid, NT, smem, s>>>(M, vin, vout, tmpV, dt, nu, ui, stage);
-  } else {
-    if (first_on_device(attr_set[0]))
-      CUP_CUDA_TRY(cudaFuncSetAttribute(k_advect_stage<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
-    ProfScope ps("advect_stage_upwind5", s);
-    k_advect_stage<0><<<grid, NT, smem, s>>>(M, vin, vout, tmpV, dt, nu, ui, stage);
-  }
-  CUP_CUDA_TRY(cudaGetLastError());
-  return 0;
 }
 
 // ---------------------------------------------------------------------------
