@@ -160,18 +160,6 @@ struct Weno {
   }
 };
 
-// Sum over a coarse face cell's four fine cells of their ghosts' tangential
-// weights: three nodes from n0 on (tan_stencil at eta = -1/4 and +1/4).
-__device__ __forceinline__ void tan_sum(int t, int& n0, double w[3]) {
-  double wa[3], wb[3];
-  const double c = t == 0 ? 0.0 : (t == BS - 1 ? 2.0 : 1.0);
-  n0 = t == 0 ? 0 : (t == BS - 1 ? BS - 3 : t - 1);
-  lagrange3(c - 0.25, wa);
-  lagrange3(c + 0.25, wb);
-#pragma unroll
-  for (int i = 0; i < 3; ++i) w[i] = wa[i] + wb[i];
-}
-
 }  // namespace
 
 template <int SCHEME>
@@ -190,7 +178,7 @@ __global__ void __launch_bounds__(AT, 4)
   const double alpha = stage == 0 ? 1.0 / 3.0 : (stage == 1 ? 15.0 / 16.0 : 8.0 / 15.0);
   const double beta = stage == 0 ? -5.0 / 9.0 : (stage == 1 ? -153.0 / 128.0 : 0.0);
   int it = 0;
-  if (int(blockIdx.x) < M.nb) meta_load(&S.meta[0], M, blockIdx.x, nullptr);
+  if (int(blockIdx.x) < M.nb) meta_load(&S.meta[0], M, blockIdx.x);
   __syncthreads();
   for (int b = blockIdx.x; b < M.nb; b += gridDim.x, ++it) {
     const StageMeta& m = S.meta[it & 1];
@@ -262,7 +250,7 @@ __global__ void __launch_bounds__(AT, 4)
         second = true;
       }
     }
-    if (b + int(gridDim.x) < M.nb) meta_issue(&S.meta[(it + 1) & 1], M, b + gridDim.x, nullptr);
+    if (b + int(gridDim.x) < M.nb) meta_issue(&S.meta[(it + 1) & 1], M, b + gridDim.x);
     cp_async_commit();
     if (threadIdx.x == 0) {  // one thread's divisions, not everybody's
       const double h = m.h, h3 = h * h * h, hf = 0.5 * h;  // h = h0 2^-level: exact

@@ -1,11 +1,5 @@
-// Asynchronous global -> shared copies for the staged block kernels:
-//   * bulk copies (cp.async.bulk, the TMA engine's 1-D form) of whole
-//     4 KB block components, completing on an mbarrier with a byte count;
-//   * per-thread 4/8-byte copies (cp.async) for scattered ghost cells and
-//     table entries, completing by commit groups.
-// Only this GPU's own memory is ever a source, and no copy is multicast.
-// Every mbarrier wait is bounded: a wait that runs out records an error and
-// returns false, so a kernel can leave instead of hanging.
+// Asynchronous global -> shared copies (cp.async): 4, 8 or 16 bytes a thread,
+// completing by commit groups.  Only this GPU's own memory is a source.
 #pragma once
 #include <stdint.h>
 
@@ -15,53 +9,6 @@ namespace cup3d {
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
-}
-
-__device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
-}
-
-// Makes initialised mbarriers visible to the asynchronous (TMA) proxy.
-__device__ __forceinline__ void mbar_init_fence() {
-  asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-}
-
-// Orders this thread's earlier generic-proxy accesses of shared memory before
-// later asynchronous-proxy (bulk copy) accesses.
-__device__ __forceinline__ void fence_proxy_async_smem() {
-  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-}
-
-__device__ __forceinline__ void mbar_arrive_expect_tx(uint64_t* bar, uint32_t bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes)
-               : "memory");
-}
-
-__device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
-  uint32_t done;
-  asm volatile(
-      "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
-      : "=r"(done)
-      : "r"(smem_u32(bar)), "r"(parity)
-      : "memory");
-  return done != 0;
-}
-
-// Polls until the phase of `parity` has completed, at most `limit` polls
-// (each try_wait itself suspends for a bounded, hardware-chosen time).
-__device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity, int limit = 1 << 22) {
-  for (int i = 0; i < limit; ++i)
-    if (mbar_try_wait(bar, parity)) return true;
-  return false;
-}
-
-// Bulk copy of `bytes` (a multiple of 16; both addresses 16-byte aligned)
-// from global to this CTA's shared memory, counted on `bar`.
-__device__ __forceinline__ void bulk_g2s(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
-  asm volatile(
-      "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_u32(dst)),
-      "l"(src), "r"(bytes), "r"(smem_u32(bar))
-      : "memory");
 }
 
 __device__ __forceinline__ void cp_async8(void* dst, const void* src) {

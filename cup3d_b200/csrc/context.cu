@@ -64,7 +64,6 @@ int ctx_upload_mesh(cup_ctx* c, int set) {
     T.arena.release();
     T.cap = 0;
     const size_t cap = size_t(m.nb) + m.nb / 4;
-    if (int rc = T.arena.alloc(&T.kerr, 1)) return rc;
     if (int rc = T.arena.alloc(&T.fk, 6 * cap)) return rc;
     if (int rc = T.arena.alloc(&T.fn, 24 * cap)) return rc;
     if (int rc = T.arena.alloc(&T.ix, 3 * cap)) return rc;
@@ -73,7 +72,6 @@ int ctx_upload_mesh(cup_ctx* c, int set) {
     T.cap = int(cap);
   }
   cudaStream_t s = c->stream;
-  CUP_CUDA_TRY(cudaMemsetAsync(T.kerr, 0, sizeof(int), s));
   CUP_CUDA_TRY(cudaMemcpyAsync(T.fk, m.face_kind.data(), 6 * size_t(m.nb) * 4, cudaMemcpyHostToDevice, s));
   CUP_CUDA_TRY(cudaMemcpyAsync(T.fn, m.face_nbr.data(), 24 * size_t(m.nb) * 4, cudaMemcpyHostToDevice, s));
   CUP_CUDA_TRY(cudaMemcpyAsync(T.ix, m.index.data(), 3 * size_t(m.nb) * 4, cudaMemcpyHostToDevice, s));
@@ -90,16 +88,7 @@ int ctx_upload_mesh(cup_ctx* c, int set) {
   c->dm.case_dt = nullptr;
   c->dm.case_sums = nullptr;
   c->dm.case_kin = nullptr;
-  c->dm.kerr = T.kerr;
   ++c->mesh_version;
-  return 0;
-}
-
-// Reads the staged kernels' error word after the stream has been synchronised.
-int ctx_check_kernels(cup_ctx* c) {
-  int e = 0;
-  CUP_CUDA_TRY(stream_d2h(c->stream, &e, c->dm.kerr, sizeof(int)));
-  if (e) return ctx_fail(c, CUP_ERR_CUDA, "stencil kernel: a wait for a block's bulk copies timed out");
   return 0;
 }
 
@@ -934,7 +923,6 @@ static int graph_capture(cup_ctx* c, int vcur, int pcur, int use_pold, cudaGraph
     CUP_CUDA_TRY(cudaMemcpyAsync(&c->gio->dt, c->d_scalars + SC_GDT, sizeof(double), cudaMemcpyDeviceToHost, s));
     CUP_CUDA_TRY(cudaMemcpyAsync(&c->gio->st, c->W.st, sizeof(KrylovState), cudaMemcpyDeviceToHost, s));
     CUP_CUDA_TRY(cudaMemcpyAsync(&c->gio->bar_error, c->W.bar_error, sizeof(int), cudaMemcpyDeviceToHost, s));
-    CUP_CUDA_TRY(cudaMemcpyAsync(&c->gio->kerr, c->dm.kerr, sizeof(int), cudaMemcpyDeviceToHost, s));
     return 0;
   };
   solver_pdl(false);
@@ -974,7 +962,6 @@ static int graph_step(cup_ctx* c, int step, double* dt_used, cup_solve_stats* st
   F.pcur = 1 - F.pcur;
   const KrylovState& K = c->gio->st;
   if (c->gio->bar_error) return ctx_fail(c, CUP_ERR_CUDA, "persistent BiCGSTAB: a grid barrier wait timed out");
-  if (c->gio->kerr) return ctx_fail(c, CUP_ERR_CUDA, "stencil kernel: a wait for a block's bulk copies timed out");
   if (dt_used) *dt_used = c->gio->dt;
   if (!(c->gio->dt > 0)) return ctx_fail(c, CUP_ERR_NAN, "dt <= 0 or NaN (Simulation.cpp:344-347)");
   float ms = 0;
@@ -1096,7 +1083,6 @@ int cup_pressure_rhs(cup_ctx* c, double dt, int32_t step) {
     return keep(c, rc);
   cudaError_t e = cudaStreamSynchronize(c->stream);
   if (e != cudaSuccess) return keep(c, set_cuda_error(e, "pressure_rhs", __FILE__, __LINE__));
-  if (int rk = ctx_check_kernels(c)) return rk;
   c->proj_open = 1;
   return 0;
 }
@@ -1117,7 +1103,7 @@ int cup_pressure_finish(cup_ctx* c, double dt, int32_t step) {
   c->proj_open = 0;
   cudaError_t e = cudaStreamSynchronize(c->stream);
   if (e != cudaSuccess) return keep(c, set_cuda_error(e, "pressure_finish", __FILE__, __LINE__));
-  return ctx_check_kernels(c);
+  return 0;
 }
 
 int cup_pressure_project(cup_ctx* c, double dt, int32_t step, cup_solve_stats* stats) {
@@ -1128,7 +1114,6 @@ int cup_pressure_project(cup_ctx* c, double dt, int32_t step, cup_solve_stats* s
   if (rc < 0) return rc;
   cudaError_t e = cudaStreamSynchronize(c->stream);
   if (e != cudaSuccess) return keep(c, set_cuda_error(e, "pressure_project", __FILE__, __LINE__));
-  if (int rk = ctx_check_kernels(c)) return rk;
   return rc;
 }
 
@@ -1165,7 +1150,6 @@ int cup_step(cup_ctx* c, int32_t step, double dt, double* dt_used, cup_solve_sta
   if (rc < 0) return rc;
   cudaError_t e = cudaStreamSynchronize(c->stream);
   if (e != cudaSuccess) return keep(c, set_cuda_error(e, "step", __FILE__, __LINE__));
-  if (int rk = ctx_check_kernels(c)) return rk;
   return rc;
 }
 

@@ -145,7 +145,6 @@ struct GraphIO {
   double cfl_fac;
   double dt;
   int bar_error;
-  int kerr;  // the staged kernels' error word
   KrylovState st;
 };
 
@@ -172,7 +171,7 @@ struct BodyState {
 struct MeshTables {
   DevArena arena;
   int cap = 0;
-  int *fk = nullptr, *fn = nullptr, *ix = nullptr, *kerr = nullptr;
+  int *fk = nullptr, *fn = nullptr, *ix = nullptr;
   int* plan = nullptr;  // 9 per block: where an adapted mesh's block takes its values from
   double* h = nullptr;
 };
@@ -271,9 +270,6 @@ int ctx_fail(cup_ctx* c, int code, const std::string& msg);
 // Uploads c->mesh into table set `set` (-1: the set in use) and points the
 // device mesh at it.
 int ctx_upload_mesh(cup_ctx* c, int set = -1);
-// CUP_ERR_CUDA with a message when a staged stencil kernel reported a timed-out
-// wait (call after synchronising the context's stream).
-int ctx_check_kernels(cup_ctx* c);
 // Room for the fields and solver work of c->mesh, all zeroed; the obstacle
 // data dropped.
 int ctx_alloc_fields(cup_ctx* c);

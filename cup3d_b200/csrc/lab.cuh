@@ -56,6 +56,19 @@ __device__ __forceinline__ void tan_stencil(int t, int half, int& n0, double w[3
   }
 }
 
+// Sum over a coarse face cell's four fine cells of their ghosts' tangential
+// weights: three nodes from n0 on (tan_stencil at eta = -1/4 and +1/4; the four fine
+// cells of one coarse cell share their nodes).
+__device__ __forceinline__ void tan_sum(int t, int& n0, double w[3]) {
+  double wa[3], wb[3];
+  const double c = t == 0 ? 0.0 : (t == BS - 1 ? 2.0 : 1.0);
+  n0 = t == 0 ? 0 : (t == BS - 1 ? BS - 3 : t - 1);
+  lagrange3(c - 0.25, wa);
+  lagrange3(c + 0.25, wb);
+#pragma unroll
+  for (int i = 0; i < 3; ++i) w[i] = wa[i] + wb[i];
+}
+
 // Ghost of a fine block at layer l (1-based) beyond its face (d, s), tangential
 // (a, bb), interpolated from the coarse neighbour cb.  get(cell of cb) reads one
 // component.  The fine block's tangential halves inside cb are (h1, h2).

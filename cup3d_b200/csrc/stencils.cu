@@ -1,14 +1,10 @@
-// Time-step stencil operators (FP64), one CTA per 8^3 block with its ghost
-// layers staged in shared memory.  Each kernel names the reference kernel it
-// computes; coarse-fine flux correction (Cubism FluxCorrection, absent from the
-// reference tree) adds, to a coarse cell next to a finer face, its own face
-// value plus the four fine face values, computed by the coarse block's CTA
-// from the fine blocks' face cells and their ghosts.
+// Pointwise time-step operators and reductions (FP64): penalization, maximum
+// velocity, per-case sums and the CFL time step.  Each kernel names the
+// reference kernel it computes.
 #include <algorithm>
 
 #include "../../include/cup3d_b200.h"
 #include "lab.cuh"
-#include "staged.cuh"
 #include "stencils.cuh"
 #include "profiler.h"
 
@@ -17,309 +13,6 @@ namespace cup3d {
 struct Vec3 {
   double v[3];
 };
-
-// lab coordinates of own face cell (layer 0) and the ghost at layer 1
-__device__ __forceinline__ void face_lab_pair(int d, int s, int a, int bb, int q[3], int g[3]) {
-  q[d] = s ? BS - 1 : 0;
-  q[tan1(d)] = a;
-  q[tan2(d)] = bb;
-  g[0] = q[0];
-  g[1] = q[1];
-  g[2] = q[2];
-  g[d] += s ? 1 : -1;
-}
-
-// ---------------------------------------------------------------------------
-// PressureProjection RHS: KernelPressureRHS (PressureProjection.cpp:96-199),
-// kernelUpdateTmpV (:202-242) and KernelDivPressure (:16-94, step > 2).
-// ---------------------------------------------------------------------------
-struct UdefGet {
-  ObstacleView ob;
-  const double* chi;
-  __device__ __forceinline__ double operator()(int c, int blk, int cell) const {
-    const int sl = ob.slot[blk];
-    if (sl < 0) return 0.0;
-    return chi[size_t(blk) * BN + cell] <= ob.chi[size_t(sl) * BN + cell]
-               ? ob.udef[(size_t(c) * ob.nslots + sl) * BN + cell]
-               : 0.0;
-  }
-};
-
-// One CTA walks its blocks through the staged pipeline (staged.cuh): the
-// velocity and p_old labs arrive by bulk copies and per-cell async copies
-// while the previous block is computed.  Blocks next to the body (rare) add
-// the u_def lab with plain loads.
-template <int USE_POLD>
-__global__ void __launch_bounds__(NT, 2)
-    k_pressure_rhs(DevMesh M, const double* __restrict__ vel, const double* __restrict__ pold,
-                   const double* __restrict__ chi, ObstacleView ob, double dt, double* __restrict__ lhs,
-                   double* __restrict__ phi) {
-  extern __shared__ __align__(16) unsigned char stage_smem[];
-  constexpr int NCH = 3 + USE_POLD;
-  using SS = StagedShape<NCH, 0>;
-  using LG = LabGeom<1>;
-  double* dlab = reinterpret_cast<double*>(stage_smem + SS::kBytes);
-  double* corr = dlab + 3 * LG::V;  // [0,512): RHS flux correction, [512,1024): div p correction
-  const size_t n = size_t(M.nb) * BN;
-  const double* src[NCH];
-#pragma unroll
-  for (int c = 0; c < NCH; ++c) src[c] = c < 3 ? vel + c * n : pold;
-  auto getV = [&](int c, int blk, int cell) { return vel[c * n + size_t(blk) * BN + cell]; };
-  auto getP = [&](int, int blk, int cell) { return pold[size_t(blk) * BN + cell]; };
-  UdefGet getD{ob, chi};
-  staged_blocks<NCH, 0>(M, src, ob.near, stage_smem, M.kerr, [&](int, int b, const StageMeta& m, double* ulab) {
-    double* plab = ulab + 3 * LG::V;
-    stage_fixup<3>(ulab, M, m, getV, true);
-    if (USE_POLD) stage_fixup<1>(plab, M, m, getP, false);
-    const bool near = m.flag != 0;
-    if (near) lab_fill<1, 3>(dlab, M, b, getD, true);
-    const bool fix = meta_has_finer(m);
-    if (fix)
-      for (int i = threadIdx.x; i < 2 * BN; i += NT) corr[i] = 0.0;
-    __syncthreads();
-    const double dtb = block_dt(M, b, dt);
-    const double h = m.h, fac = 0.5 * h * h / dtb;
-    auto U = [&](int c, int x, int y, int z) { return ulab[c * LG::V + LG::at(x, y, z)]; };
-    auto D = [&](int c, int x, int y, int z) { return near ? dlab[c * LG::V + LG::at(x, y, z)] : 0.0; };
-    auto P = [&](int x, int y, int z) { return plab[LG::at(x, y, z)]; };
-    if (fix) {
-      for (int f = 0; f < 6; ++f) {
-        if (m.kind[f] != K_FINER) continue;
-        const int d = f >> 1, s = f & 1;
-        if (threadIdx.x < 64) {
-          const int a = threadIdx.x & 7, bb = threadIdx.x >> 3;
-          int q[3], g[3];
-          face_lab_pair(d, s, a, bb, q, g);
-          const int ch = m.nbr[4 * f + (a >> 2) + 2 * (bb >> 2)];
-          const double hf = M.h[ch], facf = 0.5 * hf * hf / dtb;
-          const int oc = face_cell(d, s, 0, a, bb);
-          const double sg = s ? -1.0 : 1.0, sgc = -sg;
-          const double cq = chi[size_t(b) * BN + oc];
-          double vr = sg * fac * (U(d, g[0], g[1], g[2]) + U(d, q[0], q[1], q[2])) -
-                      sg * cq * fac * (D(d, g[0], g[1], g[2]) + D(d, q[0], q[1], q[2]));
-          double vp = USE_POLD ? h * (P(q[0], q[1], q[2]) - P(g[0], g[1], g[2])) : 0.0;
-#pragma unroll
-          for (int e2 = 0; e2 < 2; ++e2)
-#pragma unroll
-            for (int e1 = 0; e1 < 2; ++e1) {
-              const int fa = 2 * (a & 3) + e1, fb = 2 * (bb & 3) + e2;
-              const int cf = face_cell(d, 1 - s, 0, fa, fb);
-              const double uf = getV(d, ch, cf);
-              const double gu = child_ghost1([&](int cell) { return getV(d, b, cell); }, M, ch, d, s, fa, fb);
-              const double cf_chi = chi[size_t(ch) * BN + cf];
-              double df = 0.0, gd = 0.0;
-              if (near) {
-                df = getD(d, ch, cf);
-                gd = child_ghost1([&](int cell) { return getD(d, b, cell); }, M, ch, d, s, fa, fb);
-              }
-              vr += sgc * facf * (gu + uf) - sgc * cf_chi * facf * (gd + df);
-              if (USE_POLD) {
-                const double pf = getP(0, ch, cf);
-                const double gp = child_ghost1([&](int cell) { return getP(0, b, cell); }, M, ch, d, s, fa, fb);
-                vp += hf * (pf - gp);
-              }
-            }
-          corr[oc] += vr;
-          corr[BN + oc] += vp;
-        }
-        __syncthreads();
-      }
-    }
-    for (int qq = 0; qq < 2; ++qq) {
-      const int cell = threadIdx.x + qq * NT;
-      const int x = cell & 7, y = (cell >> 3) & 7, z = cell >> 6;
-      const size_t gi = size_t(b) * BN + cell;
-      double p = fac * (U(0, x + 1, y, z) - U(0, x - 1, y, z) + U(1, x, y + 1, z) - U(1, x, y - 1, z) +
-                        U(2, x, y, z + 1) - U(2, x, y, z - 1));
-      if (near) {
-        const double divUs = D(0, x + 1, y, z) - D(0, x - 1, y, z) + D(1, x, y + 1, z) - D(1, x, y - 1, z) +
-                             D(2, x, y, z + 1) - D(2, x, y, z - 1);
-        p += -chi[gi] * fac * divUs;
-      }
-      if (fix) p += corr[cell];
-      if (USE_POLD) {
-        double dp = h * (P(x + 1, y, z) + P(x - 1, y, z) + P(x, y + 1, z) + P(x, y - 1, z) + P(x, y, z + 1) +
-                         P(x, y, z - 1) - 6.0 * P(x, y, z));
-        if (fix) dp += corr[BN + cell];
-        p -= dp;
-      }
-      lhs[gi] = p;
-      phi[gi] = 0.0;
-    }
-    __syncthreads();
-  });
-}
-
-// CTAs of a staged kernel that fit on the device at once: the pipeline wants
-// one resident wave of CTAs, each walking several blocks.
-template <class K>
-static int resident_ctas(K kern, size_t smem, unsigned long long& cached_mask, int* cache) {
-  int dev = 0;
-  CUP_CUDA_TRY(cudaGetDevice(&dev));
-  if (dev < 0 || dev > 63) return set_error(CUP_ERR_ARG, "device ordinal above 63");
-  if (first_on_device(cached_mask)) {
-    int per_sm = 0, sms = 0;
-    CUP_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
-    CUP_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, NT, smem));
-    CUP_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    if (per_sm < 1) return set_error(CUP_ERR_CUDA, "staged stencil kernel does not fit on an SM");
-    cache[dev] = per_sm * sms;
-  }
-  return 0;
-}
-
-template <int USE_POLD>
-constexpr size_t rhs_smem() {
-  return StagedShape<3 + USE_POLD, 0>::kBytes + (3 * LabGeom<1>::V + 2 * BN) * sizeof(double);
-}
-
-int launch_pressure_rhs(const DevMesh& M, const double* vel, const double* pold, const double* chi,
-                        const ObstacleView& ob, double dt, int step, int step_2nd_start, double* lhs, double* phi,
-                        int grid, cudaStream_t s) {
-  static unsigned long long attr[2] = {0, 0};
-  static int resident[2][64];
-  int dev = 0;
-  CUP_CUDA_TRY(cudaGetDevice(&dev));
-  ProfScope ps("pressure_rhs", s);
-  // with udef = 0 in every slot the near-body terms (chi times the
-  // divergence of udef, with its flux correction) are exact zeros: no block
-  // needs the udef lab
-  ObstacleView o = ob;
-  if (o.udef_zero) o.near = nullptr;
-  if (step > step_2nd_start) {
-    if (int rc = resident_ctas(k_pressure_rhs<1>, rhs_smem<1>(), attr[1], resident[1])) return rc;
-    grid = std::max(1, std::min({grid, resident[1][dev], M.nb}));
-    k_pressure_rhs<1><<<grid, NT, rhs_smem<1>(), s>>>(M, vel, pold, chi, o, dt, lhs, phi);
-  } else {
-    if (int rc = resident_ctas(k_pressure_rhs<0>, rhs_smem<0>(), attr[0], resident[0])) return rc;
-    grid = std::max(1, std::min({grid, resident[0][dev], M.nb}));
-    k_pressure_rhs<0><<<grid, NT, rhs_smem<0>(), s>>>(M, vel, pold, chi, o, dt, lhs, phi);
-  }
-  CUP_CUDA_TRY(cudaGetLastError());
-  return 0;
-}
-
-// ---------------------------------------------------------------------------
-// Mean removal + incremental pressure (PressureProjection.cpp:404-446) fused
-// with KernelGradP (:244-323) and the velocity update (:451-467).  The
-// pressure p = phi - avg (+ p_old) is formed at the point of use from the
-// staged phi and p_old labs; the velocity comes in with them as interiors.
-// ---------------------------------------------------------------------------
-template <int USE_POLD>
-__global__ void __launch_bounds__(NT, 3)
-    k_grad_update(DevMesh M, double* vel, const double* __restrict__ phi, const double* __restrict__ pold,
-                  double* __restrict__ pnew, const double* sums, double dt) {
-  extern __shared__ __align__(16) unsigned char stage_smem[];
-  constexpr int NCH = 1 + USE_POLD;
-  using SS = StagedShape<NCH, 3>;
-  using LG = LabGeom<1>;
-  double* corr = reinterpret_cast<double*>(stage_smem + SS::kBytes);  // 3 BN
-  const size_t n = size_t(M.nb) * BN;
-  const double* src[NCH + 3];
-#pragma unroll
-  for (int c = 0; c < NCH; ++c) src[c] = c == 0 ? phi : pold;
-#pragma unroll
-  for (int c = 0; c < 3; ++c) src[NCH + c] = vel + c * n;
-  auto getPhi = [&](int, int blk, int cell) { return phi[size_t(blk) * BN + cell]; };
-  auto getPold = [&](int, int blk, int cell) { return pold[size_t(blk) * BN + cell]; };
-  staged_blocks<NCH, 3>(M, src, nullptr, stage_smem, M.kerr, [&](int, int b, const StageMeta& m, double* st) {
-    double* flab = st;
-    double* olab = st + LG::V;
-    const double* vin = st + NCH * LG::V;
-    const double avg = M.case_sums ? M.case_sums[2 * M.bcase[b]] / M.case_sums[2 * M.bcase[b] + 1]
-                                   : (sums ? sums[0] / sums[1] : 0.0);
-    // the pressure of any cell of the mesh (coarse-fine flux correction)
-    auto getP = [&](int, int blk, int cell) {
-      const size_t i = size_t(blk) * BN + cell;
-      const double p = phi[i] - avg;
-      return USE_POLD ? p + pold[i] : p;
-    };
-    stage_fixup<1>(flab, M, m, getPhi, false);
-    if (USE_POLD) stage_fixup<1>(olab, M, m, getPold, false);
-    const bool fix = meta_has_finer(m);
-    if (fix)
-      for (int i = threadIdx.x; i < 3 * BN; i += NT) corr[i] = 0.0;
-    __syncthreads();
-    const double dtb = block_dt(M, b, dt);
-    const double h = m.h, fac = -0.5 * dtb * h * h;
-    auto P = [&](int x, int y, int z) {
-      const int i = LG::at(x, y, z);
-      const double p = flab[i] - avg;
-      return USE_POLD ? p + olab[i] : p;
-    };
-    if (fix) {
-      for (int f = 0; f < 6; ++f) {
-        if (m.kind[f] != K_FINER) continue;
-        const int d = f >> 1, s = f & 1;
-        if (threadIdx.x < 64) {
-          const int a = threadIdx.x & 7, bb = threadIdx.x >> 3;
-          int q[3], g[3];
-          face_lab_pair(d, s, a, bb, q, g);
-          const int ch = m.nbr[4 * f + (a >> 2) + 2 * (bb >> 2)];
-          const double hf = M.h[ch], facf = -0.5 * dtb * hf * hf;
-          const double sg = s ? -1.0 : 1.0, sgc = -sg;
-          double v = sg * fac * (P(g[0], g[1], g[2]) + P(q[0], q[1], q[2]));
-#pragma unroll
-          for (int e2 = 0; e2 < 2; ++e2)
-#pragma unroll
-            for (int e1 = 0; e1 < 2; ++e1) {
-              const int fa = 2 * (a & 3) + e1, fb = 2 * (bb & 3) + e2;
-              const int cf = face_cell(d, 1 - s, 0, fa, fb);
-              const double pf = getP(0, ch, cf);
-              const double gp = child_ghost1([&](int cell) { return getP(0, b, cell); }, M, ch, d, s, fa, fb);
-              v += sgc * facf * (gp + pf);
-            }
-          corr[d * BN + face_cell(d, s, 0, a, bb)] += v;
-        }
-        __syncthreads();
-      }
-    }
-    const double ih3 = 1.0 / (h * h * h);
-    for (int qq = 0; qq < 2; ++qq) {
-      const int cell = threadIdx.x + qq * NT;
-      const int x = cell & 7, y = (cell >> 3) & 7, z = cell >> 6;
-      const size_t gi = size_t(b) * BN + cell;
-      double g0 = fac * (P(x + 1, y, z) - P(x - 1, y, z));
-      double g1 = fac * (P(x, y + 1, z) - P(x, y - 1, z));
-      double g2 = fac * (P(x, y, z + 1) - P(x, y, z - 1));
-      if (fix) {
-        g0 += corr[cell];
-        g1 += corr[BN + cell];
-        g2 += corr[2 * BN + cell];
-      }
-      vel[gi] = vin[cell] + ih3 * g0;
-      vel[n + gi] = vin[BN + cell] + ih3 * g1;
-      vel[2 * n + gi] = vin[2 * BN + cell] + ih3 * g2;
-      pnew[gi] = P(x, y, z);
-    }
-    __syncthreads();
-  });
-}
-
-template <int USE_POLD>
-constexpr size_t grad_smem() {
-  return StagedShape<1 + USE_POLD, 3>::kBytes + 3 * BN * sizeof(double);
-}
-
-int launch_grad_update(const DevMesh& M, double* vel, const double* phi, const double* pold, double* pnew,
-                       const double* sums, double dt, int step, int step_2nd_start, int grid, cudaStream_t s) {
-  static unsigned long long attr[2] = {0, 0};
-  static int resident[2][64];
-  int dev = 0;
-  CUP_CUDA_TRY(cudaGetDevice(&dev));
-  ProfScope ps("grad_update", s);
-  if (step > step_2nd_start) {
-    if (int rc = resident_ctas(k_grad_update<1>, grad_smem<1>(), attr[1], resident[1])) return rc;
-    grid = std::max(1, std::min({grid, resident[1][dev], M.nb}));
-    k_grad_update<1><<<grid, NT, grad_smem<1>(), s>>>(M, vel, phi, pold, pnew, sums, dt);
-  } else {
-    if (int rc = resident_ctas(k_grad_update<0>, grad_smem<0>(), attr[0], resident[0])) return rc;
-    grid = std::max(1, std::min({grid, resident[0][dev], M.nb}));
-    k_grad_update<0><<<grid, NT, grad_smem<0>(), s>>>(M, vel, phi, pold, pnew, sums, dt);
-  }
-  CUP_CUDA_TRY(cudaGetLastError());
-  return 0;
-}
 
 // ---------------------------------------------------------------------------
 // Penalization: KernelPenalization (Penalization.cpp:56-89) on obstacle blocks

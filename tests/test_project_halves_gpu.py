@@ -1,0 +1,68 @@
+"""The projection's two stencil passes against the CPU oracle where the
+half-block warps can go wrong: coarse-fine faces in every direction with and
+without walls, a body whose deformation velocity is not zero next to level
+changes (set through cup_set_obstacle), a non-zero pressure mean, meshes of
+one block (its own neighbour) and of odd block counts.
+
+Tolerance: 1e-12 of the largest value, FP64 on both sides with other
+summation orders (as the operator tests of test_stencils_gpu.py).
+"""
+import numpy as np
+import pytest
+
+import cup3d_b200 as cup
+import oracle
+from tests.meshes import cell_centres, make_ctx, oracle_mesh
+
+pytestmark = pytest.mark.gpu
+
+BOXES = {"one_block": "-bpdx 1 -bpdy 1 -bpdz 1 -BC_x periodic -BC_y periodic -BC_z periodic",
+         "odd_walls": "-bpdx 3 -bpdy 1 -bpdz 5 -BC_x wall -BC_y periodic -BC_z freespace"}
+
+
+def _ctx(name):
+    if name not in BOXES:
+        ctx = make_ctx(name, device=0)
+        return ctx, oracle_mesh(ctx)
+    cfg = cup.config(BOXES[name] + " -levelMax 1 -extent 1", device=0)
+    ctx = cup.Context(cfg)
+    ctx.set_mesh_uniform()
+    level, index, _ = ctx.blocks()
+    return ctx, oracle.Mesh(level, index, list(cfg.bpd), cfg.level_max, list(cfg.bc), cfg.extent)
+
+
+def _close(a, b):
+    assert np.abs(a - b).max() < 1e-12 * np.abs(b).max()
+
+
+@pytest.mark.parametrize("body", [False, True])
+@pytest.mark.parametrize("step", [1, 5])
+@pytest.mark.parametrize("name", ["one_block", "odd_walls", "amr2_free", "amr3_mixed", "amr3_periodic"])
+def test_projection_passes_match_oracle(name, step, body):
+    ctx, m = _ctx(name)
+    n = ctx.nb * 512
+    rng = np.random.default_rng(11)
+    vel, pold, phi = rng.standard_normal(3 * n), rng.standard_normal(n), 3.0 + rng.standard_normal(n)
+    obst = {}
+    if body:  # every other block holds obstacle cells with a deformation velocity
+        blocks = np.arange(0, ctx.nb, 2, dtype=np.int32)
+        ns = len(blocks)
+        chi = rng.uniform(0, 1, n)
+        chi_o = chi.reshape(-1, 512)[blocks] + 0.2 * rng.choice([-1.0, 1.0], (ns, 512))  # some cells not the body's
+        udef = rng.standard_normal(3 * ns * 512)
+        ctx.set_obstacle(blocks, chi_o.reshape(-1), udef, np.zeros(9))
+        ctx.upload("chi", chi)
+        slot = -np.ones(ctx.nb, np.int32)
+        slot[blocks] = np.arange(ns)
+        obst = dict(chi=chi, slot=slot, chi_o=chi_o.reshape(-1), udef_o=udef)
+    dt = 0.1 * m.hmin
+    ctx.upload("vel", vel)
+    ctx.upload("pres", pold)
+    ctx.pressure_rhs(dt, step)
+    _close(ctx.download("lhs"), m.pressure_rhs(vel, pold, dt, step, **obst))
+    ctx.upload("pres", phi)
+    ctx.pressure_finish(dt, step)
+    h3 = cell_centres(ctx)[1] ** 3
+    pres = phi - np.sum(phi * h3) / np.sum(h3) + (pold if step > 2 else 0.0)
+    _close(ctx.download("pres"), pres)
+    _close(ctx.download("vel"), m.grad_update(vel, pres, dt))
