@@ -122,17 +122,19 @@ static int batch_coarse_setup(cup_ctx* c, cup_ctx* const* cases) {
   for (int k = 0; k < c->ncase; ++k) {
     const long long n = c->case_first[k + 1] - c->case_first[k];
     off[k] = total;
-    total += n * n;
+    total += n * coarse_ld(int(n));
   }
   DevArena& A = c->bcoarse_arena;
   float* inv = nullptr;
   long long* d_off = nullptr;
-  double *rc = nullptr, *rc2 = nullptr, *w = nullptr;
+  double *rc = nullptr, *rc2 = nullptr, *yc = nullptr, *yc2 = nullptr, *w = nullptr;
   const int nb = c->mesh.nb;
   if (int rc_ = A.alloc(&inv, size_t(total))) return rc_;
   if (int rc_ = A.alloc(&d_off, size_t(c->ncase))) return rc_;
   if (int rc_ = A.alloc(&rc, size_t(nb))) return rc_;
   if (int rc_ = A.alloc(&rc2, size_t(nb))) return rc_;
+  if (int rc_ = A.alloc(&yc, size_t(nb))) return rc_;
+  if (int rc_ = A.alloc(&yc2, size_t(nb))) return rc_;
   if (int rc_ = A.alloc(&w, size_t(nb))) return rc_;
   CUP_CUDA_TRY(stream_h2d(c->stream, d_off, off.data(), off.size() * sizeof(long long)));
   std::vector<double> hw(nb);
@@ -143,11 +145,11 @@ static int batch_coarse_setup(cup_ctx* c, cup_ctx* const* cases) {
     if (int rc_ = coarse_build(s)) return rc_;
     const long long n = c->case_first[k + 1] - c->case_first[k];
     if (s->coarse.nb != n) return set_error(CUP_ERR_STATE, "batch two-level: a case's coarse space does not match");
-    CUP_CUDA_TRY(cudaMemcpyAsync(inv + off[k], s->coarse.inv, size_t(n * n) * sizeof(float), cudaMemcpyDeviceToDevice,
-                                 s->stream));
+    CUP_CUDA_TRY(cudaMemcpyAsync(inv + off[k], s->coarse.inv, size_t(n * coarse_ld(int(n))) * sizeof(float),
+                                 cudaMemcpyDeviceToDevice, s->stream));
     CUP_CUDA_TRY(cudaStreamSynchronize(s->stream));
   }
-  c->bcoarse = BatchCoarse{inv, d_off, rc, rc2, w};
+  c->bcoarse = BatchCoarse{inv, d_off, rc, rc2, yc, yc2, w};
   return 0;
 }
 

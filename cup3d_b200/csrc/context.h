@@ -117,10 +117,11 @@ struct CoarseSpace {
   int nb = 0;                   // blocks it was built for (0: not built)
   int mesh_version = -1;        // cup_ctx::mesh_version it was built for
   int colours = 0;              // colours of the set-up
-  float* inv = nullptr;         // A_c^-1, nb x nb, row-major, FP32 (a preconditioner needs no more)
+  float* inv = nullptr;         // A_c^-1, nb rows of coarse_ld(nb), FP32 (a preconditioner needs no more)
   double* rc = nullptr;         // nb: restricted vector
   double* rc2 = nullptr;        // nb: the second one of the persistent solver
   double* yc = nullptr;         // nb: coarse correction
+  double* yc2 = nullptr;        // nb: the second one of the persistent solver
   double* w = nullptr;          // nb: 512 h^3 of each block
   // set-up scratch: A_c (FP64, then its inverse in place), colours, block sums,
   // the per-colour neighbour map (jcap entries)
@@ -134,7 +135,7 @@ struct CoarseSpace {
   std::vector<double> host_ac;  // A_c (row-major), for checks (kept when keep_host)
   bool keep_host = false;
   int pivoted = 0;              // A_c^-1 came from the column-wise pivoted Gauss-Jordan
-  CoarseView view() const { return CoarseView{nb, inv, rc, rc2, yc, w}; }
+  CoarseView view() const { return CoarseView{nb, inv, rc, rc2, yc, yc2, w}; }
 };
 
 // Offsets into cup_ctx::d_scalars

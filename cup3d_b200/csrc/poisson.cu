@@ -19,6 +19,7 @@
 #include <cmath>
 #include <cstring>
 
+#include "async_copy.cuh"
 #include "fd.cuh"
 #include "group.cuh"
 #include "lmap.cuh"
@@ -103,9 +104,41 @@ __device__ __forceinline__ TaylorTerms cf_terms(Layer L, int u, int v) {
 // may also combine stored vectors at the point of use.
 // ---------------------------------------------------------------------------
 template <class T>
+struct Vec2;
+template <>
+struct Vec2<double> {
+  using type = double2;
+};
+template <>
+struct Vec2<float> {
+  using type = float2;
+};
+
+// Two consecutive values from an even index on (vectors start on 16-byte boundaries).
+template <class T>
+__device__ __forceinline__ double2 ld_pair(const T* v, size_t i) {
+  const typename Vec2<T>::type p = *reinterpret_cast<const typename Vec2<T>::type*>(v + i);
+  return make_double2(double(p.x), double(p.y));
+}
+
+// block(b): what the accessor adds to the cells of block b (nothing for a
+// stored vector); pair(i, block(b)): the values at i and i + 1 (i even).
+template <class T>
 struct VecAt {
   const T* v;
   __device__ __forceinline__ double operator()(size_t i) const { return double(ld_stream(v + i)); }
+  __device__ __forceinline__ double2 block(int) const { return make_double2(0.0, 0.0); }
+  __device__ __forceinline__ double2 pair(size_t i, double2) const { return ld_pair(v, i); }
+};
+
+// The same for a caller's vector of any alignment (8 bytes).
+struct VecAtAny {
+  const double* v;
+  __device__ __forceinline__ double operator()(size_t i) const { return ld_stream(v + i); }
+  __device__ __forceinline__ double2 block(int) const { return make_double2(0.0, 0.0); }
+  __device__ __forceinline__ double2 pair(size_t i, double2) const {
+    return make_double2(ld_stream(v + i), ld_stream(v + i + 1));
+  }
 };
 
 // Group-cooperative copy of block b's table entries into bi (the caller
@@ -124,48 +157,104 @@ __device__ __forceinline__ void fill_block_info(const DevMesh& M, int b, BlockIn
   }
 }
 
-// Flux across coarse-fine face f into face cell (a, bb) of block b
-// (PoissonSolverExp::makeFlux, PoissonSolverExp.cpp:157-219): the fine side
-// of a coarser face (coarse layer staged in tile.cl[f]), or the four fine
-// fluxes of a finer face (Taylor terms from the block's own layer).  Reads
-// the tile after the group barrier that follows its filling.
+// The fine cells at face cell (a, bb) of finer face f, layers 0 (close) and 1
+// (far): four 16-byte pairs of the child (x faces: a pair holds both layers; y
+// and z faces: two neighbours of one layer).
 template <class X>
-__device__ __forceinline__ double cf_flux(const BlockInfo& bi, const X& x, const GroupTile& tile, int f, int kind,
-                                          int a, int bb) {
+__device__ __forceinline__ void fine_load(const BlockInfo& bi, const X& x, int f, int a, int bb, double2 (&p)[4]) {
+  const int d = f >> 1, s = f & 1, lo_a = 2 * (a & 3), lo_b = 2 * (bb & 3);
+  const int ch = bi.nbr[4 * f + (a >> 2) + 2 * (bb >> 2)];
+  const double2 k = x.block(ch);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int l = s ? i >> 1 : 7 - (i >> 1), q = i & 1;
+    const int cell = d == 0   ? (lo_b + (i >> 1)) * 64 + (lo_a + q) * 8 + (s ? 0 : 6)
+                     : d == 1 ? (lo_b + q) * 64 + l * 8 + lo_a
+                              : l * 64 + (lo_b + q) * 8 + lo_a;
+    p[i] = x.pair(size_t(ch) * BN + cell, k);
+  }
+}
+
+// Flux across finer face f into face cell (a, bb) (PoissonSolverExp::makeFlux,
+// PoissonSolverExp.cpp:157-219): the four fine fluxes, with the Taylor terms
+// of the block's own layer.  p: the fine cells (fine_load).
+__device__ __forceinline__ double finer_flux(const BlockInfo& bi, const GroupTile& tile, int f, int a, int bb,
+                                             const double2 (&p)[4]) {
   const int d = f >> 1, s = f & 1;
   auto own = [&](int cell) { return tile.v[cell >> 6][((cell >> 3) & 7) + 1][(cell & 7) + 1]; };
-  const double h = bi.h;
-  if (kind == K_COARSER) {
-    const double* cl = tile.cl[f];
-    auto L = [&](int u, int v) { return d == 1 ? cl[v + 8 * u] : cl[u + 8 * v]; };
-    const int h1 = (bi.par >> tan1(d)) & 1, h2 = (bi.par >> tan2(d)) & 1;
-    const int c1 = h1 * 4 + (a >> 1), c2 = h2 * 4 + (bb >> 1);
-    const double sa = (a & 1) ? 1.0 : -1.0, sb = (bb & 1) ? 1.0 : -1.0;
-    const TaylorTerms Tt = d == 1 ? cf_terms(L, c2, c1) : cf_terms(L, c1, c2);
-    const double tay = d == 1 ? Tt.at(sb, sa) : Tt.at(sa, sb);
-    const double xs = own(face_cell(d, s, 0, a, bb)), xi = own(face_cell(d, s, 1, a, bb));
-    return h * (2. / 3. * xs - 1. / 5. * xi + 8. / 15. * tay - xs);
-  }
   auto L = [&](int u, int v) { return d == 1 ? own(face_cell(d, s, 0, v, u)) : own(face_cell(d, s, 0, u, v)); };
   const TaylorTerms Tt = d == 1 ? cf_terms(L, bb, a) : cf_terms(L, a, bb);
-  const int ch = bi.nbr[4 * f + (a >> 2) + 2 * (bb >> 2)];
-  const double hf = 0.5 * h;  // h = h0 2^-level: exact
-  const size_t xc = size_t(ch) * BN;
-  double close[4], far[4];
-#pragma unroll
-  for (int q4 = 0; q4 < 4; ++q4) {
-    const int fa = 2 * (a & 3) + (q4 & 1), fb = 2 * (bb & 3) + (q4 >> 1);
-    close[q4] = x(xc + face_cell(d, 1 - s, 0, fa, fb));
-    far[q4] = x(xc + face_cell(d, 1 - s, 1, fa, fb));
-  }
+  const double hf = 0.5 * bi.h;  // h = h0 2^-level: exact
   double acc = 0.0;
 #pragma unroll
   for (int q4 = 0; q4 < 4; ++q4) {
     const double sa = (q4 & 1) ? 1.0 : -1.0, sb = (q4 >> 1) ? 1.0 : -1.0;
     const double tay = d == 1 ? Tt.at(sb, sa) : Tt.at(sa, sb);
-    acc += hf * (close[q4] - (2. / 3. * close[q4] - 1. / 5. * far[q4] + 8. / 15. * tay));
+    const double lo = (q4 & 1) ? p[q4 >> 1].y : p[q4 >> 1].x, hi = (q4 & 1) ? p[2 + (q4 >> 1)].y : p[2 + (q4 >> 1)].x;
+    const double close = d ? lo : (s ? p[q4].x : p[q4].y), far = d ? hi : (s ? p[q4].y : p[q4].x);
+    acc += hf * (close - (2. / 3. * close - 1. / 5. * far + 8. / 15. * tay));
   }
   return acc;
+}
+
+// The fluxes of face cell (gx, gy) go to tile.cl, where the owners pick them up.
+// The finer faces (bits of `finer`), one after the other (two at a time would
+// share a round trip, but spill 400 bytes a thread on every block's path).
+template <class X>
+__device__ __forceinline__ void finer_fluxes(const BlockInfo* b, const X x, GroupTile* t, unsigned finer) {
+  const BlockInfo& bi = *b;
+  GroupTile& tile = *t;
+  const GroupIdx G;
+  while (finer) {
+    const int f = __ffs(finer) - 1;
+    finer &= finer - 1;
+    double2 p[4];
+    fine_load(bi, x, f, G.gx, G.gy, p);
+    tile.cl[f][G.lane] = finer_flux(bi, tile, f, G.gx, G.gy, p);
+  }
+}
+
+// The coarser faces (bits of `coarser`, whose coarse layers are in tile.cl).
+// Thread 16 i + j forms the Taylor terms of coarse cell j of the quarter that
+// the block covers on the i-th of them; its four values there replace the
+// layer in tile.cl, and every thread takes its face cell's.  Out of line: its
+// registers would be taken from every block's path.
+__device__ __noinline__ void coarser_fluxes(const BlockInfo* b, GroupTile* tl, unsigned coarser) {
+  const BlockInfo& bi = *b;
+  GroupTile& tile = *tl;
+  const GroupIdx G;
+  int f = -1;
+  unsigned m = coarser;
+  for (int i = 0; m; ++i, m &= m - 1)
+    if (i == (G.lane >> 4)) f = __ffs(m) - 1;
+  const int j = G.lane & 15;
+  double t[4];
+  if (f >= 0) {
+    const int d = f >> 1;
+    const double* cl = tile.cl[f];
+    auto L = [&](int u, int v) { return d == 1 ? cl[v + 8 * u] : cl[u + 8 * v]; };
+    const int c1 = 4 * ((bi.par >> tan1(d)) & 1) + (j & 3), c2 = 4 * ((bi.par >> tan2(d)) & 1) + (j >> 2);
+    const TaylorTerms Tt = d == 1 ? cf_terms(L, c2, c1) : cf_terms(L, c1, c2);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const double sa = (q & 1) ? 1.0 : -1.0, sb = (q >> 1) ? 1.0 : -1.0;
+      t[q] = d == 1 ? Tt.at(sb, sa) : Tt.at(sa, sb);
+    }
+  }
+  __syncwarp();  // the face's 16 threads have read its layer
+  if (f >= 0) {
+    double* cl = tile.cl[f];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) cl[2 * (j & 3) + (q & 1) + 8 * (2 * (j >> 2) + (q >> 1))] = t[q];
+  }
+  group_sync(G.g);
+  for (m = coarser; m; m &= m - 1) {
+    const int fc = __ffs(m) - 1, d = fc >> 1, s = fc & 1;
+    auto own = [&](int cell) { return tile.v[cell >> 6][((cell >> 3) & 7) + 1][(cell & 7) + 1]; };
+    const double xs = own(face_cell(d, s, 0, G.gx, G.gy)), xi = own(face_cell(d, s, 1, G.gx, G.gy));
+    const double tay = tile.cl[fc][G.lane];
+    tile.cl[fc][G.lane] = bi.h * (2. / 3. * xs - 1. / 5. * xi + 8. / 15. * tay - xs);
+  }
 }
 
 template <class T>
@@ -176,9 +265,13 @@ __device__ __forceinline__ void load_col(const T* __restrict__ v, int b, const G
 }
 
 // y = A x on the thread's column of block b (col = x there, already loaded).
-// Same-level and boundary faces from the tile and halos; coarse-fine faces:
-// each thread computes the flux of one face cell per face, owners add them.
-// Ends with a group barrier (tile free for reuse).
+// Same-level and boundary faces from the tile and halos.  Coarse-fine faces
+// take as few round trips as they can, for the blocks that have them set the
+// length of the phase (17 of 21 us in the solver's first one on the sphere
+// mesh, where a block without takes 5): a finer face's cells come in 16-byte
+// pairs, and the Taylor terms of all coarser faces (three at most: a block's other three face
+// neighbours are its siblings) are formed at once, 16 coarse cells a face.  Each thread computes the flux of one face cell per face; the owners
+// add them.  Ends with a group barrier (tile free for reuse).
 template <class X>
 __device__ __forceinline__ void spmv_group(const BlockInfo& bi, const X& x, const double col[8], double ms,
                                            int mean_mode, GroupTile& tile, const GroupIdx& G, double y[8]) {
@@ -195,7 +288,7 @@ __device__ __forceinline__ void spmv_group(const BlockInfo& bi, const X& x, cons
   // face-local cell (gx, gy) of each.  The ghost of a same-level face is the
   // neighbour's face cell; on any other face it is the block's own face cell
   // (zero flux; coarse-fine faces get their flux below).
-  bool cf = false;
+  unsigned coarser = 0, finer = 0;
 #pragma unroll
   for (int f = 0; f < 6; ++f) {
     const int d = f >> 1, s = f & 1;
@@ -206,27 +299,22 @@ __device__ __forceinline__ void spmv_group(const BlockInfo& bi, const X& x, cons
       double* ghost = d == 0 ? &tile.v[G.gy][G.gx + 1][s ? BS + 1 : 0] : &tile.v[G.gy][s ? BS + 1 : 0][G.gx + 1];
       *ghost = x(src);
     }
-    if (kind[f] == K_COARSER)
+    if (kind[f] == K_COARSER) {
       tile.cl[f][G.lane] = x(size_t(fn[4 * f]) * BN + face_cell(d, 1 - s, 0, G.gx, G.gy));
-    cf |= kind[f] >= K_COARSER;
+      coarser |= 1u << f;
+    }
+    if (kind[f] == K_FINER) finer |= 1u << f;
   }
 #pragma unroll
   for (int z = 0; z < 8; ++z) tile.v[z][G.gy + 1][G.gx + 1] = col[z];
+  const bool cf = (coarser | finer) != 0;  // uniform per block
   group_sync(G.g);
   double zf0 = 0.0, zf1 = 0.0;  // z-face fluxes of the own column (cells z = 0, 7)
-  if (cf) {                      // uniform per block
-#pragma unroll 1
-    for (int f = 0; f < 6; ++f) {
-      const int kf = bi.kind[f];
-      if (kf < K_COARSER) continue;
-      const double fl = cf_flux(bi, x, tile, f, kf, G.gx, G.gy);
-      if (f < 4)
-        tile.flx[f][G.lane] = fl;
-      else if (f == 4)
-        zf0 = fl;
-      else
-        zf1 = fl;
-    }
+  if (cf) {
+    if (finer) finer_fluxes(&bi, x, &tile, finer);
+    if (coarser) coarser_fluxes(&bi, &tile, coarser);
+    zf0 = tile.cl[4][G.lane];
+    zf1 = tile.cl[5][G.lane];
     group_sync(G.g);
   }
   const double h = bi.h;
@@ -252,11 +340,11 @@ __device__ __forceinline__ void spmv_group(const BlockInfo& bi, const X& x, cons
       } else if (f < 2) {
         if (G.gx == (s ? 7 : 0))
 #pragma unroll
-          for (int z = 0; z < 8; ++z) y[z] += tile.flx[f][G.gy + 8 * z];
+          for (int z = 0; z < 8; ++z) y[z] += tile.cl[f][G.gy + 8 * z];
       } else {
         if (G.gy == (s ? 7 : 0))
 #pragma unroll
-          for (int z = 0; z < 8; ++z) y[z] += tile.flx[f][G.gx + 8 * z];
+          for (int z = 0; z < 8; ++z) y[z] += tile.cl[f][G.gx + 8 * z];
       }
     }
   }
@@ -315,7 +403,7 @@ __global__ void __launch_bounds__(NT) k_spmv(DevMesh M, const double* __restrict
     load_col(x, b, G, col);
     fill_block_info(M, b, tiles[G.g].bi, G.lane);
     group_sync(G.g);
-    spmv_group(tiles[G.g].bi, VecAt<double>{x}, col, ms, mean_mode, tiles[G.g], G, out);
+    spmv_group(tiles[G.g].bi, VecAtAny{x}, col, ms, mean_mode, tiles[G.g], G, out);
     double* yb = y + size_t(b) * BN + G.gy * 8 + G.gx;
 #pragma unroll
     for (int z = 0; z < 8; ++z) yb[z * 64] = out[z];
@@ -366,26 +454,17 @@ struct KArgs {
   // two-level preconditioner (persistent solver): A_c^-1 (cnb x cnb, cnb = 0:
   // none), the restricted vectors of zv and zr and the blocks' 512 h^3
   int cnb;           // single case: blocks of A_c; batch: 1 when the cases carry coarse spaces
-  const long long* coff;  // batch: offset of each case's A_c^-1 (nb_c x nb_c) in cinv; null: one case
+  const long long* coff;  // batch: offset of each case's A_c^-1 (nb_c rows of coarse_ld(nb_c)) in cinv; null: one case
   const float* cinv;
   double* crc_v;
   double* crc_r;
+  double* cyc_v;  // per block: the coarse corrections of zv and zr
+  double* cyc_r;
   const double* cw;
   // learned local map (persistent solver, lmap.cuh): W in fragment order
   // (null: none) and the [nb][896] BF16 lab buffer
   const uint4* lw;
   uint16_t* llab;
-};
-
-template <class T>
-struct Vec2;
-template <>
-struct Vec2<double> {
-  using type = double2;
-};
-template <>
-struct Vec2<float> {
-  using type = float2;
 };
 
 template <class T>
@@ -794,13 +873,34 @@ __global__ void __launch_bounds__(NT) k_bicg_e(KArgs<T> A) {
 // written only in another phase, so no phase needs a second buffer.  The
 // scalars, the restart rule and the stopping tests are fin_a..fin_e's.
 // ---------------------------------------------------------------------------
-template <class T>
-struct Comb2At {  // a + c b
+// COARSE: zr and zv are stored without the coarse correction of a block's
+// cells, one value per block, which is added (and rounded to T) where they are
+// read: adding it to the stored vectors took a pass over each of them per
+// iteration.
+template <class T, bool COARSE>
+struct Comb2At {  // (a + ya) + c (b + yb), ya and yb per block
   const T* a;
   const T* b;
   double c;
-  __device__ __forceinline__ double operator()(size_t i) const {
-    return double(ld_stream(a + i)) + c * double(ld_stream(b + i));
+  const double* ya;
+  const double* yb;  // null: none
+  __device__ __forceinline__ double2 block(int blk) const {
+    return COARSE ? make_double2(ya[blk], yb ? yb[blk] : 0.0) : make_double2(0.0, 0.0);
+  }
+  __device__ __forceinline__ double sum(double u, double v, double2 k) const {
+    if (COARSE) {
+      u = double(T(u + k.x));
+      if (yb) v = double(T(v + k.y));
+    }
+    return u + c * v;
+  }
+  __device__ __forceinline__ double cell(size_t i, double2 k) const {
+    return sum(double(ld_stream(a + i)), double(ld_stream(b + i)), k);
+  }
+  __device__ __forceinline__ double operator()(size_t i) const { return cell(i, block(int(i / BN))); }
+  __device__ __forceinline__ double2 pair(size_t i, double2 k) const {
+    const double2 u = ld_pair(a, i), v = ld_pair(b, i);
+    return make_double2(sum(u.x, v.x, k), sum(u.y, v.y, k));
   }
 };
 
@@ -900,39 +1000,72 @@ __device__ __forceinline__ void coarse_restrict(const double c[8], double* rc, i
   if (G.lane == 0) rc[b] = s[0];
 }
 
-// row: block b's row of A_c^-1 (n entries), rc: the restriction of the
-// blocks that row spans.
-template <class T>
-__device__ __forceinline__ double coarse_block_row(const KArgs<T>& A, const GroupIdx& G, int b, const float* row,
-                                                   const double* rc, int n, T* v, double* gsm) {
-  double s[1] = {0.0};
-  for (int j = G.lane; j < n; j += GROUP) s[0] += double(row[j]) * __ldcg(rc + j);
-  group_reduce<1>(s, gsm, G);
-  const double yc = s[0];
-  double c[8];
-  load_col(v, b, G, c);
+// Rows r0 and r1 of A_c^-1 (FP32) times the restriction rc (shared memory, or
+// global where it does not fit) onto s: lane l of the group takes columns l,
+// l + 64, ..., and COARSE_AHEAD loads of each row are in flight.
+constexpr int COARSE_AHEAD = 20;
+__device__ __forceinline__ void coarse_rows(const float* r0, const float* r1, const double* rc, int n, int lane,
+                                            double (&s)[2]) {
+#pragma unroll 1
+  for (int j0 = lane; j0 < n; j0 += GROUP * COARSE_AHEAD) {
+    float a[COARSE_AHEAD], b[COARSE_AHEAD];
 #pragma unroll
-  for (int z = 0; z < 8; ++z) c[z] = double(T(c[z] + yc));
-  store_col(v, b, G, c);
-  return G.lane == 0 ? yc * A.cw[b] : 0.0;  // summed over the CTA's threads by the grid reduction
+    for (int q = 0; q < COARSE_AHEAD; ++q) {  // no branch: it would end the batch of loads
+      const int j = min(j0 + GROUP * q, n - 1);
+      a[q] = r0[j];
+      b[q] = r1[j];
+    }
+#pragma unroll
+    for (int q = 0; q < COARSE_AHEAD; ++q) {
+      const int j = j0 + GROUP * q;
+      if (j < n) {
+        const double c = rc[j];
+        s[0] += double(a[q]) * c;
+        s[1] += double(b[q]) * c;
+      }
+    }
+  }
 }
 
-template <class T>
-__device__ __forceinline__ double coarse_block(const KArgs<T>& A, const GroupIdx& G, int b, const double* rc, T* v,
-                                               double* gsm) {
-  return coarse_block_row(A, G, b, A.cinv + size_t(b) * A.cnb, rc, A.cnb, v, gsm);
-}
-
-// The same in a batch: block b of case c (blocks cf .. cf + n - 1), whose
-// A_c^-1 starts at coff[c] of the packed, block-diagonal cinv.
-template <class T>
-__device__ __forceinline__ double coarse_block_case(const KArgs<T>& A, const GroupIdx& G, int b, int cf, int n,
-                                                    long long off, const double* rc, T* v, double* gsm) {
-  return coarse_block_row(A, G, b, A.cinv + off + size_t(b - cf) * n, rc + cf, n, v, gsm);
+// The coarse corrections of a group's blocks block(0) .. block(nblk - 1):
+// yc[b] = row b of A_c^-1 times rc, two rows at a time.  cf: the first block
+// that the rows span, n their length.  With the learned map (lw), which adds
+// to the stored vector v, the corrections are added to v instead and yc stays
+// zero.  Returns the sum of yc 512 h^3, the corrections' part of sum(v h^3),
+// in lane 0 (0 elsewhere; the reductions sum over the threads).
+template <class T, class Block>
+__device__ __forceinline__ double coarse_blocks(const KArgs<T>& A, const GroupIdx& G, int nblk, Block block,
+                                                const double* rc, int cf, int n, const float* inv, double* yc, T* v,
+                                                double* gsm) {
+  const int ld = coarse_ld(n);
+  double added = 0.0;
+#pragma unroll 1
+  for (int k = 0; k < nblk; k += 2) {
+    const int b0 = block(k), b1 = block(min(k + 1, nblk - 1));
+    double s[2] = {0.0, 0.0};
+    coarse_rows(inv + size_t(b0 - cf) * ld, inv + size_t(b1 - cf) * ld, rc, n, G.lane, s);
+    group_reduce<2>(s, gsm, G);
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      if (k + i >= nblk) break;
+      const int b = i ? b1 : b0;
+      if (A.lw) {
+        double c[8];
+        load_col(v, b, G, c);
+#pragma unroll
+        for (int z = 0; z < 8; ++z) c[z] = double(T(c[z] + s[i]));
+        store_col(v, b, G, c);
+      } else if (G.lane == 0) {
+        yc[b] = s[i];
+      }
+      if (G.lane == 0) added += __dmul_rn(s[i], A.cw[b]);
+    }
+  }
+  return added;
 }
 
 // P0 (once): zr = M^-1 r for the initial residual; sum(zr h^3)
-template <class T>
+template <class T, bool COARSE>
 __device__ __forceinline__ double p0_block(const KArgs<T>& A, const GroupIdx& G, GroupTile& tile,
                                            const BlockInfo& bi, const double* inv) {
   FdTile& ftile = reinterpret_cast<FdTile&>(tile);
@@ -940,7 +1073,7 @@ __device__ __forceinline__ double p0_block(const KArgs<T>& A, const GroupIdx& G,
   const double h = bi.h;
   double c[8];
   load_col(A.r, b, G, c);
-  if (A.cnb) coarse_restrict(c, A.crc_r, b, ftile.v[0][0] + 0, G);
+  if (COARSE) coarse_restrict(c, A.crc_r, b, ftile.v[0][0] + 0, G);
   block_inverse_group(c, ftile, G, h, inv);
   double s = 0.0;
 #pragma unroll
@@ -954,19 +1087,20 @@ __device__ __forceinline__ double p0_block(const KArgs<T>& A, const GroupIdx& G,
 
 // P1: z1 = zr + beta q (beta = 0 after a restart, which also sets rhat = r);
 //     nu = A z1; zv = M^-1 nu; (rhat, nu), sum(zv h^3)
-template <class T>
+template <class T, bool COARSE>
 __device__ __forceinline__ void p1_block(const KArgs<T>& A, const GroupIdx& G, GroupTile& tile, const BlockInfo& bi,
                                          const double* inv, double beta, double ms, bool restart,
                                          double (&acc)[2]) {
   FdTile& ftile = reinterpret_cast<FdTile&>(tile);
-  const Comb2At<T> z1{A.z1, A.p, beta};
+  const Comb2At<T, COARSE> z1{A.z1, A.p, beta, A.cyc_r, nullptr};
   const int b = bi.id;
   const double h = bi.h;
   double col[8], y[8], rh[8];
   {
     const size_t o = size_t(b) * BN + G.gy * 8 + G.gx;
+    const double2 k = z1.block(b);
 #pragma unroll
-    for (int z = 0; z < 8; ++z) col[z] = z1(o + z * 64);  // the accessor the ghosts use: the same values
+    for (int z = 0; z < 8; ++z) col[z] = z1.cell(o + z * 64, k);  // the accessor the ghosts use: the same values
   }
   spmv_group(bi, z1, col, ms, A.mean_mode, tile, G, y);
   if (restart) {
@@ -981,7 +1115,7 @@ __device__ __forceinline__ void p1_block(const KArgs<T>& A, const GroupIdx& G, G
     acc[0] += rh[z] * y[z];
   }
   store_col(A.nu, b, G, y);
-  if (A.cnb) coarse_restrict(y, A.crc_v, b, ftile.v[0][0] + 0, G);
+  if (COARSE) coarse_restrict(y, A.crc_v, b, ftile.v[0][0] + 0, G);
   block_inverse_group(y, ftile, G, h, inv);
   double s = 0.0;
 #pragma unroll
@@ -994,16 +1128,17 @@ __device__ __forceinline__ void p1_block(const KArgs<T>& A, const GroupIdx& G, G
 }
 
 // P2: t = A (zr - alpha zv); s = r - alpha nu; (t, s), (t, t)
-template <class T>
+template <class T, bool COARSE>
 __device__ __forceinline__ void p2_block(const KArgs<T>& A, const GroupIdx& G, GroupTile& tile, const BlockInfo& bi,
                                          double alpha, double ms, double (&acc)[2]) {
-  const Comb2At<T> z2{A.z1, A.z2, -alpha};
+  const Comb2At<T, COARSE> z2{A.z1, A.z2, -alpha, A.cyc_r, A.cyc_v};
   const int b = bi.id;
   double col[8], y[8];
   {
     const size_t o = size_t(b) * BN + G.gy * 8 + G.gx;
+    const double2 k = z2.block(b);
 #pragma unroll
-    for (int z = 0; z < 8; ++z) col[z] = z2(o + z * 64);  // the accessor the ghosts use: the same values
+    for (int z = 0; z < 8; ++z) col[z] = z2.cell(o + z * 64, k);  // the accessor the ghosts use: the same values
   }
   spmv_group(bi, z2, col, ms, A.mean_mode, tile, G, y);
   double r[8], nu[8];
@@ -1021,7 +1156,7 @@ __device__ __forceinline__ void p2_block(const KArgs<T>& A, const GroupIdx& G, G
 
 // P3: x_new = x + alpha z1 + omega z2; r = s - omega t; q = z1 - omega zv;
 //     zr = M^-1 r; (rhat, r), (r, r), sum(zr h^3), sum(q h^3)
-template <class T>
+template <class T, bool COARSE>
 __device__ __forceinline__ void p3_block(const KArgs<T>& A, const GroupIdx& G, GroupTile& tile, const BlockInfo& bi,
                                          const double* inv, const T* xc, T* xn, double alpha, double beta,
                                          double omega, double (&acc)[4]) {
@@ -1050,8 +1185,13 @@ __device__ __forceinline__ void p3_block(const KArgs<T>& A, const GroupIdx& G, G
     load_col(A.p, b, G, q);
     load_col(A.z2, b, G, zv);
     load_col(xc, b, G, x);
+    const double yr = COARSE ? A.cyc_r[b] : 0.0, yv = COARSE ? A.cyc_v[b] : 0.0;
 #pragma unroll
     for (int z = 0; z < 8; ++z) {
+      if (COARSE) {
+        zr[z] = double(T(zr[z] + yr));
+        zv[z] = double(T(zv[z] + yv));
+      }
       const double z1 = zr[z] + beta * q[z], z2 = zr[z] - alpha * zv[z];
       x[z] = double(T((x[z] + alpha * z1) + omega * z2));
       q[z] = double(T(z1 - omega * zv[z]));
@@ -1060,7 +1200,7 @@ __device__ __forceinline__ void p3_block(const KArgs<T>& A, const GroupIdx& G, G
     store_col(xn, b, G, x);
     store_col(A.p, b, G, q);
   }
-  if (A.cnb) coarse_restrict(rn, A.crc_r, b, ftile.v[0][0] + 0, G);
+  if (COARSE) coarse_restrict(rn, A.crc_r, b, ftile.v[0][0] + 0, G);
   block_inverse_group(rn, ftile, G, h, inv);
   double s = 0.0;
 #pragma unroll
@@ -1084,22 +1224,24 @@ __device__ __forceinline__ void p3_block(const KArgs<T>& A, const GroupIdx& G, G
 constexpr size_t kSmemCache = BN * sizeof(double);
 constexpr size_t kSmemTiles = kSmemCache + PGROUPS * KB_CACHE * sizeof(BlockInfo);
 constexpr size_t kPersistentSmem = kSmemTiles + PGROUPS * sizeof(GroupTile);
+// columns of the restriction that the coarse phase stages at once, over the tiles
+constexpr int kStageCols = int(PGROUPS * sizeof(GroupTile) / sizeof(double)) & ~63;
 constexpr size_t kLearnedSmem = std::max(kPersistentSmem, kSmemTiles + LMAP_TILE_BYTES);
 static_assert(kSmemTiles % 16 == 0, "tiles and staged labs start 16-byte aligned");
 static_assert(LMAP_GATHER * sizeof(LabMeta) <= PGROUPS * sizeof(GroupTile), "the gather's table entries fit in the tiles");
 static_assert(PNT == 256, "the learned map's phases run on 8 warps (4 groups of 64 threads)");
 
-template <class T>
+template <class T, bool COARSE>
 __global__ void __launch_bounds__(PNT, 8 / PGROUPS) k_bicg_persistent(KArgs<T> A, GridSync Gs) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   double* inv_eig = reinterpret_cast<double*>(smem_raw);
   BlockInfo* cache = reinterpret_cast<BlockInfo*>(smem_raw + kSmemCache);
   GroupTile* tiles = reinterpret_cast<GroupTile*>(smem_raw + kSmemTiles);
-  __shared__ double red[64];
+  __shared__ double red[128];
   __shared__ KrylovState S;
   __shared__ double ms_zr;  // sum(zr h^3) of the current zr
   __shared__ unsigned int epoch;
-  __shared__ double gred[2 * PGROUPS];  // per-group reduction scratch of the coarse phases
+  __shared__ double gred[4 * PGROUPS];  // per-group reduction scratch of the coarse phases
   const GroupIdx G;
   const DevMesh& M = A.M;
   GroupTile& tile = tiles[G.g];
@@ -1114,6 +1256,9 @@ __global__ void __launch_bounds__(PNT, 8 / PGROUPS) k_bicg_persistent(KArgs<T> A
     epoch = 0u;
   }
   __syncthreads();
+  if (COARSE && A.lw)  // the corrections go into the vectors themselves
+    PERSISTENT_BLOCKS(bi)
+      if (G.lane == 0) A.cyc_v[bi.id] = A.cyc_r[bi.id] = 0.0;
   bool ok = true;
   // PREP and INIT: x0's mean row and sum(x0 h^3); r = b - A x0, rhat = r,
   // p = 0 and the scalars of iteration 0
@@ -1136,14 +1281,29 @@ __global__ void __launch_bounds__(PNT, 8 / PGROUPS) k_bicg_persistent(KArgs<T> A
   // The parts of the preconditioner that need the whole vector v (nu or r)
   // in place, added to its block part z (zv or zr):
   //   * the coarse correction of the two-level preconditioner, from v's
-  //     restriction rc: every group adds it on its blocks;
+  //     restriction rc: every group forms its blocks' values yc;
   //   * the learned local map (lmap.cuh): the CTAs gather v's labs, then,
   //     after a grid barrier, the GEMM adds W lab / h.
   // The grid sum of the added sum(z h^3) comes back in every CTA.  One grid
   // barrier, two with the learned map.
-  auto extra_phases = [&](const double* rc, const T* v, T* z, double& added) -> bool {
+  const int gslot = blockIdx.x * PGROUPS + G.g, gstep = gridDim.x * PGROUPS;
+  const int gblk = gslot < M.nb ? (M.nb - 1 - gslot) / gstep + 1 : 0;  // the group's blocks
+  auto group_block = [&](int k) { return M.order ? M.order[gslot + k * gstep] : gslot + k * gstep; };
+  auto extra_phases = [&](const double* rc, double* yc, const T* v, T* z, double& added) -> bool {
     double a[1] = {0.0};
-    if (A.cnb) PERSISTENT_BLOCKS(bi) a[0] += coarse_block<T>(A, G, bi.id, rc, z, &gred[2 * G.g]);
+    if (COARSE) {
+      // rc into the tiles, one copy for the CTA's groups (a copy a group reads
+      // the same lines of L2 four times as often)
+      double* st = reinterpret_cast<double*>(smem_raw + kSmemTiles);
+      __syncthreads();
+      const bool staged = A.cnb <= kStageCols;
+      if (staged)
+        for (int j = threadIdx.x; j < A.cnb; j += PNT) cp_async8(st + j, rc + j);
+      cp_async_commit();
+      cp_async_wait<0>();
+      __syncthreads();
+      a[0] += coarse_blocks<T>(A, G, gblk, group_block, staged ? st : rc, 0, A.cnb, A.cinv, yc, z, &gred[4 * G.g]);
+    }
     if (A.lw) {
       __syncthreads();  // the groups are done with their tiles
       lmap_gather<T>(M, v, A.llab, reinterpret_cast<LabMeta*>(smem_raw + kSmemTiles), mean_blk);
@@ -1157,13 +1317,13 @@ __global__ void __launch_bounds__(PNT, 8 / PGROUPS) k_bicg_persistent(KArgs<T> A
     }
     return true;
   };
-  const bool extra = A.cnb || A.lw;
+  const bool extra = COARSE || A.lw;
   if (ok && !S.done) {
     double a[1] = {0.0};
-    PERSISTENT_BLOCKS(bi) a[0] += p0_block<T>(A, G, tile, bi, inv_eig);
+    PERSISTENT_BLOCKS(bi) a[0] += p0_block<T, COARSE>(A, G, tile, bi, inv_eig);
     ok = grid_allreduce<1>(a, Gs, epoch, red);
     double cz = 0.0;
-    if (ok && extra) ok = extra_phases(A.crc_r, A.r, A.z1, cz);
+    if (ok && extra) ok = extra_phases(A.crc_r, A.cyc_r, A.r, A.z1, cz);
     // q = 0 at the start (init_block), so z1 = zr
     if (threadIdx.x == 0) ms_zr = S.mean_sum = a[0] + cz;
     __syncthreads();
@@ -1172,7 +1332,7 @@ __global__ void __launch_bounds__(PNT, 8 / PGROUPS) k_bicg_persistent(KArgs<T> A
     const bool restart = S.restart_pending != 0;
     const double beta = restart ? 0.0 : S.beta;
     double a[2] = {0.0, 0.0};
-    PERSISTENT_BLOCKS(bi) p1_block<T>(A, G, tile, bi, inv_eig, beta, S.mean_sum, restart, a);
+    PERSISTENT_BLOCKS(bi) p1_block<T, COARSE>(A, G, tile, bi, inv_eig, beta, S.mean_sum, restart, a);
     if (!(ok = grid_allreduce<2>(a, Gs, epoch, red))) break;
     if (threadIdx.x == 0) {
       fin_a(S, S.mean_sum, restart);
@@ -1183,18 +1343,18 @@ __global__ void __launch_bounds__(PNT, 8 / PGROUPS) k_bicg_persistent(KArgs<T> A
     __syncthreads();
     if (extra) {  // zv += the rest of M^-1 nu; sum(z2 h^3) with it
       double cv = 0.0;
-      if (!(ok = extra_phases(A.crc_v, A.nu, A.z2, cv))) break;
+      if (!(ok = extra_phases(A.crc_v, A.cyc_v, A.nu, A.z2, cv))) break;
       if (threadIdx.x == 0) S.mean_sum = ms_zr - S.alpha * (a[1] + cv);
       __syncthreads();
     }
     double d[2] = {0.0, 0.0};
-    PERSISTENT_BLOCKS(bi) p2_block<T>(A, G, tile, bi, S.alpha, S.mean_sum, d);
+    PERSISTENT_BLOCKS(bi) p2_block<T, COARSE>(A, G, tile, bi, S.alpha, S.mean_sum, d);
     if (!(ok = grid_allreduce<2>(d, Gs, epoch, red))) break;
     if (threadIdx.x == 0) fin_d(S, d);
     __syncthreads();
     double e[4] = {0.0, 0.0, 0.0, 0.0};
     PERSISTENT_BLOCKS(bi)
-        p3_block<T>(A, G, tile, bi, inv_eig, xslot(A, S.cur), xslot(A, S.nxt), S.alpha, S.beta, S.omega, e);
+        p3_block<T, COARSE>(A, G, tile, bi, inv_eig, xslot(A, S.cur), xslot(A, S.nxt), S.alpha, S.beta, S.omega, e);
     if (!(ok = grid_allreduce<4>(e, Gs, epoch, red))) break;
     if (threadIdx.x == 0) {
       const double re[2] = {e[0], e[1]};
@@ -1206,7 +1366,7 @@ __global__ void __launch_bounds__(PNT, 8 / PGROUPS) k_bicg_persistent(KArgs<T> A
     __syncthreads();
     if (extra && !S.done) {  // zr += the rest of M^-1 r; the sums with it
       double cr = 0.0;
-      if (!(ok = extra_phases(A.crc_r, A.r, A.z1, cr))) break;
+      if (!(ok = extra_phases(A.crc_r, A.cyc_r, A.r, A.z1, cr))) break;
       if (threadIdx.x == 0) {
         ms_zr = e[2] + cr;
         S.mean_sum = S.restart_pending ? ms_zr : ms_zr + S.beta * e[3];
@@ -1390,7 +1550,7 @@ __device__ __forceinline__ void batch_fill_cache(const DevMesh& M, const BatchAr
 #define BATCH_BLOCKS(bi) \
   for (int k_ = 0; k_ < P.nblk; ++k_) if (const BlockInfo& bi = batch_block(M, B, cache, tile, P, k_, G); true)
 
-template <class T>
+template <class T, bool COARSE>
 __global__ void __launch_bounds__(PNT, 8 / PGROUPS) k_bicg_batched(KArgs<T> A, GridSync Gs, BatchArgs B) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   double* inv_eig = reinterpret_cast<double*>(smem_raw);
@@ -1422,15 +1582,24 @@ __global__ void __launch_bounds__(PNT, 8 / PGROUPS) k_bicg_batched(KArgs<T> A, G
   __syncthreads();
   // the case's first group writes its state and done flag
   auto lead = [&]() { return P.c >= 0 && gidx == gfirst[P.c] && G.lane == 0; };
-  // two-level preconditioner: the coarse correction of each running case on
-  // v (zr or zv) from its restriction rc, added by the case's groups; the
-  // case's added sum(v h^3) comes back to its groups (one more barrier)
-  auto coarse_phase = [&](const double* rc, T* v, bool active, double& added) -> bool {
+  // two-level preconditioner: the coarse corrections yc of each running
+  // case's blocks (of zr or zv) from the restriction rc, formed by the case's
+  // groups; their part of sum(z h^3) comes back to them (one more barrier)
+  auto group_block = [&](int k) { return B.cblocks[B.cfirst[P.c] + P.j + k * P.ng]; };
+  auto coarse_phase = [&](const double* rc, double* yc, bool active, double& added) -> bool {
     double a[1] = {0.0};
     if (active) {
       const int cf = B.cfirst[P.c], n = B.cfirst[P.c + 1] - cf;
-      const long long off = A.coff[P.c];
-      BATCH_BLOCKS(bi) a[0] += coarse_block_case<T>(A, G, bi.id, cf, n, off, rc, v, gsm);
+      const bool staged = n <= int(sizeof(GroupTile) / sizeof(double));
+      double* st = reinterpret_cast<double*>(&tile);
+      group_sync(G.g);
+      if (staged)
+        for (int j = G.lane; j < n; j += GROUP) cp_async8(st + j, rc + cf + j);
+      cp_async_commit();
+      cp_async_wait<0>();
+      group_sync(G.g);
+      a[0] += coarse_blocks<T>(A, G, P.nblk, group_block, staged ? st : rc + cf, cf, n, A.cinv + A.coff[P.c], yc,
+                               static_cast<T*>(nullptr), gsm);
     }
     const bool okc = batch_allreduce<1, false>(a, B, Gs, epoch, gsm, G, gidx, P.c, gfirst[max(P.c, 0)],
                                                gfirst[max(P.c, 0) + 1], nullptr);
@@ -1457,11 +1626,11 @@ __global__ void __launch_bounds__(PNT, 8 / PGROUPS) k_bicg_batched(KArgs<T> A, G
   }
   if (ok) {
     double a[1] = {0.0};
-    if (P.c >= 0 && !S.done) BATCH_BLOCKS(bi) a[0] += p0_block<T>(A, G, tile, bi, inv_eig);
+    if (P.c >= 0 && !S.done) BATCH_BLOCKS(bi) a[0] += p0_block<T, COARSE>(A, G, tile, bi, inv_eig);
     ok = batch_allreduce<1, false>(a, B, Gs, epoch, gsm, G, gidx, P.c, gfirst[max(P.c, 0)], gfirst[max(P.c, 0) + 1],
                                    nullptr);
     double cz = 0.0;
-    if (ok && A.cnb) ok = coarse_phase(A.crc_r, A.z1, P.c >= 0 && !S.done, cz);
+    if (ok && COARSE) ok = coarse_phase(A.crc_r, A.cyc_r, P.c >= 0 && !S.done, cz);
     // q = 0 at the start, so z1 = zr
     if (ok && P.c >= 0 && G.lane == 0) S.ms_zr = S.mean_sum = a[0] + cz;
     if (ok && lead()) {
@@ -1475,7 +1644,7 @@ __global__ void __launch_bounds__(PNT, 8 / PGROUPS) k_bicg_batched(KArgs<T> A, G
     bool restart = active && S.restart_pending != 0;
     double beta = restart ? 0.0 : S.beta;
     double a[2] = {0.0, 0.0};
-    if (active) BATCH_BLOCKS(bi) p1_block<T>(A, G, tile, bi, inv_eig, beta, S.mean_sum, restart, a);
+    if (active) BATCH_BLOCKS(bi) p1_block<T, COARSE>(A, G, tile, bi, inv_eig, beta, S.mean_sum, restart, a);
     // the groups that did P1 for case c: this pass's deal
     for (int i = threadIdx.x; i <= B.ncase; i += blockDim.x) gfirst_prev[i] = gfirst[i];
     __syncthreads();
@@ -1525,21 +1694,21 @@ __global__ void __launch_bounds__(PNT, 8 / PGROUPS) k_bicg_batched(KArgs<T> A, G
       S.mean_sum = S.ms_zr - S.alpha * a[1];  // sum(z2 h^3)
     }
     __syncthreads();
-    if (A.cnb) {  // zv += the coarse correction of nu; sum(z2 h^3) with it
+    if (COARSE) {  // zv += the coarse correction of nu; sum(z2 h^3) with it
       double cv = 0.0;
-      if (!(ok = coarse_phase(A.crc_v, A.z2, active, cv))) break;
+      if (!(ok = coarse_phase(A.crc_v, A.cyc_v, active, cv))) break;
       if (active && G.lane == 0) S.mean_sum = S.ms_zr - S.alpha * (a[1] + cv);
       __syncthreads();
     }
     const int g0 = gfirst[max(P.c, 0)], g1 = gfirst[max(P.c, 0) + 1];
     double d[2] = {0.0, 0.0};
-    if (active) BATCH_BLOCKS(bi) p2_block<T>(A, G, tile, bi, S.alpha, S.mean_sum, d);
+    if (active) BATCH_BLOCKS(bi) p2_block<T, COARSE>(A, G, tile, bi, S.alpha, S.mean_sum, d);
     if (!(ok = batch_allreduce<2, false>(d, B, Gs, epoch, gsm, G, gidx, P.c, g0, g1, nullptr))) break;
     if (active && G.lane == 0) fin_d(S, d);
     __syncthreads();
     double e[4] = {0.0, 0.0, 0.0, 0.0};
     if (active)
-      BATCH_BLOCKS(bi) p3_block<T>(A, G, tile, bi, inv_eig, xslot(A, S.cur), xslot(A, S.nxt), S.alpha, S.beta,
+      BATCH_BLOCKS(bi) p3_block<T, COARSE>(A, G, tile, bi, inv_eig, xslot(A, S.cur), xslot(A, S.nxt), S.alpha, S.beta,
                                    S.omega, e);
     if (!(ok = batch_allreduce<4, false>(e, B, Gs, epoch, gsm, G, gidx, P.c, g0, g1, nullptr))) break;
     if (active && G.lane == 0) {
@@ -1549,9 +1718,9 @@ __global__ void __launch_bounds__(PNT, 8 / PGROUPS) k_bicg_batched(KArgs<T> A, G
       S.mean_sum = S.restart_pending ? e[2] : e[2] + S.beta * e[3];  // sum(z1 h^3) of the next P1
     }
     __syncthreads();
-    if (A.cnb) {  // zr += the coarse correction of r; the sums with it
+    if (COARSE) {  // zr += the coarse correction of r; the sums with it
       double cr = 0.0;
-      if (!(ok = coarse_phase(A.crc_r, A.z1, active && !S.done, cr))) break;
+      if (!(ok = coarse_phase(A.crc_r, A.cyc_r, active && !S.done, cr))) break;
       if (active && !S.done && G.lane == 0) {
         S.ms_zr = e[2] + cr;
         S.mean_sum = S.restart_pending ? S.ms_zr : S.ms_zr + S.beta * e[3];
@@ -1678,6 +1847,7 @@ static KArgs<T> make_args(const DevMesh& M, const T* b, T* x, T* const v[9], Poi
   A.cinv = nullptr;
   A.coff = nullptr;
   A.crc_v = A.crc_r = nullptr;
+  A.cyc_v = A.cyc_r = nullptr;
   A.cw = nullptr;
   A.lw = nullptr;
   A.llab = nullptr;
@@ -1746,10 +1916,14 @@ static cudaError_t launch_pdl(void (*kern)(KArgs<T>), int grid, cudaStream_t s, 
 // reduction buffer.
 template <class T>
 static int persistent_grid(int nb, const PoissonWork& W, int* grid, size_t dyn = kPersistentSmem) {
-  void (*kern)(KArgs<T>, GridSync) = k_bicg_persistent<T>;
-  CUP_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(dyn)));
-  int per_sm = 0, dev = 0, sms = 0;
-  CUP_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, PNT, dyn));
+  int per_sm = 8, dev = 0, sms = 0;
+  // every CTA resident with and without the coarse correction alike
+  for (auto kern : {k_bicg_persistent<T, false>, k_bicg_persistent<T, true>}) {
+    int n = 0;
+    CUP_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kLearnedSmem)));
+    CUP_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, PNT, dyn));
+    per_sm = std::min(per_sm, n);
+  }
   CUP_CUDA_TRY(cudaGetDevice(&dev));
   CUP_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
   if (per_sm < 1) return set_error(CUP_ERR_CUDA, "persistent BiCGSTAB: kernel does not fit on an SM");
@@ -1775,18 +1949,23 @@ int persistent_solver_groups(int nb, PoissonWork& W, int* groups) {
   return 0;
 }
 
+// The arrival counter and the error flag start at zero.
+static int grid_sync_reset(PoissonWork& W, cudaStream_t s) {
+  CUP_CUDA_TRY(cudaMemsetAsync(W.bar, 0, sizeof(unsigned int), s));
+  CUP_CUDA_TRY(cudaMemsetAsync(W.bar_error, 0, sizeof(int), s));
+  return 0;
+}
+
 // Launches the persistent solver: one cooperative grid (every CTA resident)
 // that runs iterations until the state says done.
 template <class T>
 static int launch_persistent(const KArgs<T>& A, PoissonWork& W, cudaStream_t s, const char* name) {
   const size_t dyn = A.lw ? kLearnedSmem : kPersistentSmem;
-  void (*kern)(KArgs<T>, GridSync) = k_bicg_persistent<T>;
+  void (*kern)(KArgs<T>, GridSync) = A.cnb ? k_bicg_persistent<T, true> : k_bicg_persistent<T, false>;
   int grid = W.pgrid;
   if (grid <= 0 || A.lw)
     if (int rc = persistent_grid<T>(A.M.nb, W, &grid, dyn)) return rc;
-  // the arrival counter and the error flag start at zero
-  CUP_CUDA_TRY(cudaMemsetAsync(W.bar, 0, sizeof(unsigned int), s));
-  CUP_CUDA_TRY(cudaMemsetAsync(W.bar_error, 0, sizeof(int), s));
+  if (int rc = grid_sync_reset(W, s)) return rc;
   GridSync Gs{W.bar, W.partial, W.bar_error, W.barrier_cycles > 0 ? W.barrier_cycles : kBarrierClockLimit};
   KArgs<T> Aa = A;
   void* args[] = {(void*)&Aa, (void*)&Gs};
@@ -1798,16 +1977,20 @@ static int launch_persistent(const KArgs<T>& A, PoissonWork& W, cudaStream_t s, 
 // CTAs and block groups of the batched solver: every CTA resident (one
 // group per block at most), the same shape as the single-case solver.
 int batch_solver_shape(int nb, int ncase, int* grid, int* groups) {
-  const size_t dyn = batch_smem(ncase);
   // every CTA resident for the FP64 solver and the FP32 inner solves alike
-  void (*kern)(KArgs<double>, GridSync, BatchArgs) = k_bicg_batched<double>;
-  void (*kernf)(KArgs<float>, GridSync, BatchArgs) = k_bicg_batched<float>;
-  CUP_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(dyn)));
-  CUP_CUDA_TRY(cudaFuncSetAttribute(kernf, cudaFuncAttributeMaxDynamicSharedMemorySize, int(dyn)));
-  int per_sm = 0, per_sm_f = 0, dev = 0, sms = 0;
-  CUP_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, PNT, dyn));
-  CUP_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_f, kernf, PNT, dyn));
-  per_sm = std::min(per_sm, per_sm_f);
+  int per_sm = 8, dev = 0, sms = 0;
+  const size_t dyn = batch_smem(ncase);
+  auto fit = [&](auto kern) -> int {
+    int n = 0;
+    CUP_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(dyn)));
+    CUP_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, PNT, dyn));
+    per_sm = std::min(per_sm, n);
+    return 0;
+  };
+  if (int rc = fit(k_bicg_batched<double, false>)) return rc;
+  if (int rc = fit(k_bicg_batched<double, true>)) return rc;
+  if (int rc = fit(k_bicg_batched<float, false>)) return rc;
+  if (int rc = fit(k_bicg_batched<float, true>)) return rc;
   CUP_CUDA_TRY(cudaGetDevice(&dev));
   CUP_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
   if (per_sm < 1) return set_error(CUP_ERR_CUDA, "batched BiCGSTAB: kernel does not fit on an SM");
@@ -1850,13 +2033,15 @@ static int batched_launch(const DevMesh& M, const T* b, T* x, T* const v[9], con
     A.coff = coarse->off;
     A.crc_v = coarse->rc;
     A.crc_r = coarse->rc2;
+    A.cyc_v = coarse->yc;
+    A.cyc_r = coarse->yc2;
     A.cw = coarse->w;
   }
   GridSync Gs{W.bar, W.partial, W.bar_error, W.barrier_cycles > 0 ? W.barrier_cycles : kBarrierClockLimit};
   BatchArgs Ba{B.cfirst, B.cblocks, B.part, B.case_done, B.ncase, B.groups};
   void* args[] = {(void*)&A, (void*)&Gs, (void*)&Ba};
   const size_t dyn = batch_smem(B.ncase);
-  void (*kern)(KArgs<T>, GridSync, BatchArgs) = k_bicg_batched<T>;
+  void (*kern)(KArgs<T>, GridSync, BatchArgs) = A.cnb ? k_bicg_batched<T, true> : k_bicg_batched<T, false>;
   if (!P.graph) CUP_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(dyn)));
   {
     ProfScope ps("bicg_batched", s);
@@ -2096,6 +2281,8 @@ static int run_bicgstab(const DevMesh& M, const T* b, T* x, T* const v[9], const
     A.cinv = coarse->inv;
     A.crc_v = coarse->rc;
     A.crc_r = coarse->rc2;
+    A.cyc_v = coarse->yc;
+    A.cyc_r = coarse->yc2;
     A.cw = coarse->w;
   }
   if (lmap) {
@@ -2301,7 +2488,8 @@ __global__ void __launch_bounds__(PNT, 8 / PGROUPS) k_pbicg_persistent(PArgs A, 
   double* inv_eig = reinterpret_cast<double*>(smem_raw);
   BlockInfo* cache = reinterpret_cast<BlockInfo*>(smem_raw + kSmemCache);
   GroupTile* tiles = reinterpret_cast<GroupTile*>(smem_raw + kSmemTiles);
-  __shared__ double red[64];
+  __shared__ double red[128];
+  __shared__ double dots[6];
   __shared__ PState S;
   __shared__ unsigned int epoch;
   const GroupIdx G;
@@ -2498,7 +2686,7 @@ __global__ void __launch_bounds__(PNT, 8 / PGROUPS) k_pbicg_persistent(PArgs A, 
       if (threadIdx.x == 0) {
         S.omega = omn;
         S.ms = d[6];
-        for (int i = 0; i < 6; ++i) red[32 + i] = d[i];
+        for (int i = 0; i < 6; ++i) dots[i] = d[i];
       }
       sync_state();
     } else {
@@ -2621,13 +2809,13 @@ __global__ void __launch_bounds__(PNT, 8 / PGROUPS) k_pbicg_persistent(PArgs A, 
       if (threadIdx.x == 0) {
         S.omega = omn;
         S.ms = d[6];
-        for (int i = 0; i < 6; ++i) red[32 + i] = d[i];
+        for (int i = 0; i < 6; ++i) dots[i] = d[i];
       }
       sync_state();
     }
     // scalars, restart, best iterate, stopping test (every CTA, its own copy)
     if (threadIdx.x == 0) {
-      const double r0r = red[32], r0w = red[33], r0s = red[34], r0z = red[35], n1 = red[36], n2 = red[37];
+      const double r0r = dots[0], r0w = dots[1], r0s = dots[2], r0z = dots[3], n1 = dots[4], n2 = dots[5];
       const double omn = S.omega;
       S.norm = sqrt(n1);
       S.beta = S.alpha / (omn + eps) * r0r / (S.r0r_prev + eps);
@@ -2743,8 +2931,7 @@ int poisson_pipelined(const DevMesh& M, const double* b, double* x, const SolveP
   CUP_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
   if (per_sm < 1) return set_error(CUP_ERR_CUDA, "pipelined BiCGSTAB: kernel does not fit on an SM");
   const int grid = std::max(1, std::min({per_sm * sms, (M.nb + PGROUPS - 1) / PGROUPS, std::max(W.grid, W.ggrid) / 2}));
-  CUP_CUDA_TRY(cudaMemsetAsync(W.bar, 0, sizeof(unsigned int), s));
-  CUP_CUDA_TRY(cudaMemsetAsync(W.bar_error, 0, sizeof(int), s));
+  if (int rc = grid_sync_reset(W, s)) return rc;
   GridSync Gs{W.bar, W.partial, W.bar_error, W.barrier_cycles > 0 ? W.barrier_cycles : kBarrierClockLimit};
   void* args[] = {(void*)&A, (void*)&Gs};
   {
