@@ -20,7 +20,7 @@ constexpr int PV = 1000;  // padded voxels
 __device__ __forceinline__ int pv(int x, int y, int z) { return (x + 1) + 10 * ((y + 1) + 10 * (z + 1)); }
 __device__ __forceinline__ int pv_of_cell(int c) { return pv(c & 7, (c >> 3) & 7, c >> 6); }
 
-struct Act {
+struct alignas(16) Act {
   uint16_t v[2][PV][8];
 };
 
@@ -106,38 +106,88 @@ __device__ void conv_cc(const Act& in, const uint16_t* Wsm, Act& out) {
       }
 }
 
-// Layer 0: 1 -> C, 'valid' 3^3 conv of the 10^3 input, into act (BF16).
-__device__ void conv_in(const float* x0, const float* W0, Act& out) {
-  for (int c = threadIdx.x; c < BN; c += blockDim.x) {
-    const int x = c & 7, y = (c >> 3) & 7, z = c >> 6;
-    float acc[CNN_C];
+// Eight BF16 values of a 16-byte word as floats, and back.
+__device__ __forceinline__ void unpack8(const uint16_t* p, float (&f)[8]) {
+  const uint4 w = *reinterpret_cast<const uint4*>(p);
+  const uint32_t u[4] = {w.x, w.y, w.z, w.w};
 #pragma unroll
-    for (int co = 0; co < CNN_C; ++co) acc[co] = 0.f;
-    for (int tap = 0; tap < 27; ++tap) {
-      const int dx = tap % 3, dy = (tap / 3) % 3, dz = tap / 9;
-      const float xv = x0[(x + dx) + 10 * ((y + dy) + 10 * (z + dz))];
+  for (int i = 0; i < 4; ++i) {
+    f[2 * i] = __uint_as_float(u[i] << 16);
+    f[2 * i + 1] = __uint_as_float(u[i] & 0xffff0000u);
+  }
+}
+__device__ __forceinline__ void pack8(uint16_t* p, const float* f) {
+  uint32_t u[4];
 #pragma unroll
-      for (int co = 0; co < CNN_C; ++co) acc[co] = fmaf(W0[co * 27 + tap], xv, acc[co]);
-    }
-    const int p = pv(x, y, z);
+  for (int i = 0; i < 4; ++i) u[i] = uint32_t(f2bf(f[2 * i])) | (uint32_t(f2bf(f[2 * i + 1])) << 16);
+  *reinterpret_cast<uint4*>(p) = make_uint4(u[0], u[1], u[2], u[3]);
+}
+
+// The 16 weights of a tap (the one-channel layers' weights are held [tap][channel]).
+__device__ __forceinline__ void tap_weights(const float* w, int tap, float (&f)[CNN_C]) {
 #pragma unroll
-    for (int co = 0; co < CNN_C; ++co) out.v[co >> 3][p][co & 7] = f2bf(acc[co]);
+  for (int i = 0; i < CNN_C; i += 4) {
+    const float4 v = *reinterpret_cast<const float4*>(w + tap * CNN_C + i);
+    f[i] = v.x;
+    f[i + 1] = v.y;
+    f[i + 2] = v.z;
+    f[i + 3] = v.w;
   }
 }
 
-// Layer 3: C -> 1, 'same' 3^3 conv, FP32 output z[512].
-__device__ void conv_out(const Act& in, const float* W3, float* z) {
-  for (int c = threadIdx.x; c < BN; c += blockDim.x) {
-    const int x = c & 7, y = (c >> 3) & 7, zz = c >> 6;
-    float acc = 0.f;
-    for (int tap = 0; tap < 27; ++tap) {
-      const int dx = tap % 3 - 1, dy = (tap / 3) % 3 - 1, dz = tap / 9 - 1;
-      const int p = pv(x + dx, y + dy, zz + dz);
+// Layer 0: 1 -> C, 'valid' 3^3 conv of the 10^3 input, into act (BF16).  Two
+// cells a thread (256 threads), so that a tap's weights are read once for
+// both; activations move as 16-byte words (one at a time, the layer's 432
+// weight reads a cell were most of its time).
+__device__ void conv_in(const float* x0, const float* W0, Act& out) {
+  static_assert(BN == 2 * NT, "two cells a thread");
+  const int x = threadIdx.x & 7, y = (threadIdx.x >> 3) & 7, z = threadIdx.x >> 6;
+  float acc[2][CNN_C];
 #pragma unroll
-      for (int ci = 0; ci < CNN_C; ++ci) acc = fmaf(W3[ci * 27 + tap], bf2f(in.v[ci >> 3][p][ci & 7]), acc);
+  for (int h = 0; h < 2; ++h)
+#pragma unroll
+    for (int co = 0; co < CNN_C; ++co) acc[h][co] = 0.f;
+#pragma unroll 1
+  for (int tap = 0; tap < 27; ++tap) {
+    const int dx = tap % 3, dy = (tap / 3) % 3, dz = tap / 9;
+    float w[CNN_C];
+    tap_weights(W0, tap, w);
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const float xv = x0[(x + dx) + 10 * ((y + dy) + 10 * (z + 4 * h + dz))];
+#pragma unroll
+      for (int co = 0; co < CNN_C; ++co) acc[h][co] = fmaf(w[co], xv, acc[h][co]);
     }
-    z[c] = acc;
   }
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const int p = pv(x, y, z + 4 * h);
+    pack8(&out.v[0][p][0], &acc[h][0]);
+    pack8(&out.v[1][p][0], &acc[h][8]);
+  }
+}
+
+// Layer 3: C -> 1, 'same' 3^3 conv, FP32 output z[512].  Two cells a thread.
+__device__ void conv_out(const Act& in, const float* W3, float* z) {
+  const int x = threadIdx.x & 7, y = (threadIdx.x >> 3) & 7, zz = threadIdx.x >> 6;
+  float acc[2] = {0.f, 0.f};
+#pragma unroll 1
+  for (int tap = 0; tap < 27; ++tap) {
+    const int dx = tap % 3 - 1, dy = (tap / 3) % 3 - 1, dz = tap / 9 - 1;
+    float w[CNN_C];
+    tap_weights(W3, tap, w);
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int p = pv(x + dx, y + dy, zz + 4 * h + dz);
+      float a[8], b[8];
+      unpack8(&in.v[0][p][0], a);
+      unpack8(&in.v[1][p][0], b);
+#pragma unroll
+      for (int ci = 0; ci < CNN_C; ++ci) acc[h] = fmaf(w[ci], ci < 8 ? a[ci] : b[ci - 8], acc[h]);
+    }
+  }
+#pragma unroll
+  for (int h = 0; h < 2; ++h) z[threadIdx.x + h * NT] = acc[h];
 }
 
 struct FwdSmem {
@@ -146,7 +196,7 @@ struct FwdSmem {
   float z[BN];
   uint16_t w1[27 * 16 * 16];
   uint16_t w2[27 * 16 * 16];
-  float w0[CNN_W0], w3[CNN_W3];
+  alignas(16) float w0[CNN_W0], w3[CNN_W3];  // [tap][channel]
   double red[64];
 };
 
@@ -156,8 +206,9 @@ __device__ void load_weights(FwdSmem& S, const CnnWeights& W) {
     S.w2[i] = W.w2_bf16[i];
   }
   const float* m = W.master;
-  for (int i = threadIdx.x; i < CNN_W0; i += blockDim.x) S.w0[i] = m[OFF_W0 + i];
-  for (int i = threadIdx.x; i < CNN_W3; i += blockDim.x) S.w3[i] = m[OFF_W3 + i];
+  // the masters are [channel][tap]
+  for (int i = threadIdx.x; i < CNN_W0; i += blockDim.x) S.w0[(i % 27) * CNN_C + i / 27] = m[OFF_W0 + i];
+  for (int i = threadIdx.x; i < CNN_W3; i += blockDim.x) S.w3[(i % 27) * CNN_C + i / 27] = m[OFF_W3 + i];
 }
 
 // full forward on S.x0 (already normalised) -> S.z; leaves L2 output in S.a
@@ -337,14 +388,51 @@ struct TrainSmem {
   float z[BN];        // output, then dL/dz
   float etmp[BN], rtmp[BN];  // residual-norm loss: error, then its block Laplacian
   uint16_t w1[27 * 256], w2[27 * 256], w1t[27 * 256], w2t[27 * 256];
-  float w0[CNN_W0], w3[CNN_W3];
+  alignas(16) float w0[CNN_W0], w3[CNN_W3];  // [tap][channel]
   float red[64];
 };
+
+// A CTA's gradient row: its first sample's gradients start it.
+__device__ __forceinline__ void add_to(float& g, float v, bool first) { g = first ? v : g + v; }
+
+// Weight gradient of a one-channel layer: gW[ch * 27 + tap] += sum over the
+// block's cells of the one-channel value f(tap, cell) times the 16 channels of
+// `act` at voxel p(tap, cell).  Eight threads a tap, each a z plane of the
+// block with all 16 channels in registers (a thread per weight read every
+// activation as a 2-byte word, 512 cells one after the other).
+template <class F, class P>
+__device__ __forceinline__ void wgrad_1c(const Act& act, F f, P p, float* gW, bool first) {
+  const int tap = threadIdx.x >> 3, z = threadIdx.x & 7;
+  float acc[CNN_C];
+#pragma unroll
+  for (int i = 0; i < CNN_C; ++i) acc[i] = 0.f;
+  if (tap < 27)
+#pragma unroll 2
+    for (int c = 64 * z; c < 64 * z + 64; ++c) {
+      const float v = f(tap, c);
+      const int q = p(tap, c);
+      float a[8], b[8];
+      unpack8(&act.v[0][q][0], a);
+      unpack8(&act.v[1][q][0], b);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        acc[i] = fmaf(a[i], v, acc[i]);
+        acc[8 + i] = fmaf(b[i], v, acc[8 + i]);
+      }
+    }
+#pragma unroll
+  for (int i = 0; i < CNN_C; ++i)
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) acc[i] += __shfl_xor_sync(0xffffffffu, acc[i], o);
+  if (tap < 27 && z == 0)
+#pragma unroll
+    for (int i = 0; i < CNN_C; ++i) add_to(gW[i * 27 + tap], acc[i], first);
+}
 
 // weight gradient of a C->C layer: dW[tap][co][ci] += sum_v in[v+tap][ci] dout[v][co].
 // Tensor cores: M = co (16), N = ci (two n8 tiles), K = voxels (32 steps of
 // 16).  Warp w handles taps w, w+8, ...
-__device__ void wgrad_cc(const Act& in, const Act& dpre, float* gW /* master layout [co][ci][tap] */) {
+__device__ void wgrad_cc(const Act& in, const Act& dpre, float* gW /* master layout [co][ci][tap] */, bool first) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int lm = lane >> 3, lr = lane & 7, g = lane >> 2, tq = lane & 3;
   for (int tap = warp; tap < 27; tap += 8) {
@@ -375,8 +463,8 @@ __device__ void wgrad_cc(const Act& in, const Act& dpre, float* gW /* master lay
 #pragma unroll
       for (int hr = 0; hr < 2; ++hr) {
         const int co = g + 8 * hr, ci = nt * 8 + 2 * tq;
-        gW[(co * 16 + ci) * 27 + tap] += acc[nt][2 * hr];
-        gW[(co * 16 + ci + 1) * 27 + tap] += acc[nt][2 * hr + 1];
+        add_to(gW[(co * 16 + ci) * 27 + tap], acc[nt][2 * hr], first);
+        add_to(gW[(co * 16 + ci + 1) * 27 + tap], acc[nt][2 * hr + 1], first);
       }
   }
 }
@@ -389,8 +477,9 @@ __device__ void load_train_weights(TrainSmem& S, const CnnWeights& W) {
     S.w2t[i] = W.w2t_bf16[i];
   }
   const float* m = W.master;
-  for (int i = threadIdx.x; i < CNN_W0; i += blockDim.x) S.w0[i] = m[OFF_W0 + i];
-  for (int i = threadIdx.x; i < CNN_W3; i += blockDim.x) S.w3[i] = m[OFF_W3 + i];
+  // the masters are [channel][tap]
+  for (int i = threadIdx.x; i < CNN_W0; i += blockDim.x) S.w0[(i % 27) * CNN_C + i / 27] = m[OFF_W0 + i];
+  for (int i = threadIdx.x; i < CNN_W3; i += blockDim.x) S.w3[(i % 27) * CNN_C + i / 27] = m[OFF_W3 + i];
 }
 
 // grad_partial row of this CTA accumulates dL/dparams over its samples.
@@ -423,18 +512,23 @@ __global__ void __launch_bounds__(NT, 1) k_cnn_train(CnnWeights W, const float* 
   TrainSmem& S = *reinterpret_cast<TrainSmem*>(smem_raw);
   load_train_weights(S, W);
   float* gp = gpart + size_t(blockIdx.x) * CNN_NPARAM;
-  if (backward)
-    for (int i = threadIdx.x; i < CNN_NPARAM; i += NT) gp[i] = 0.f;
+  if (backward)  // the bias slots stay zero; the weights' start with the first sample
+    for (int i = threadIdx.x; i < CNN_NPARAM; i += NT)
+      if (!((i >= OFF_W0 && i < OFF_B0) || (i >= OFF_W1 && i < OFF_B1) || (i >= OFF_W2 && i < OFF_B2) ||
+            (i >= OFF_W3 && i < OFF_B3)))
+        gp[i] = 0.f;
+  // the layers write the interiors only: the borders stay zero
+  zero_act(S.a1);
+  zero_act(S.a2);
+  zero_act(S.a3);
+  zero_act(S.d);
+  zero_act(S.e);
   float loss = 0.f;
   for (int sidx = blockIdx.x; sidx < n; sidx += gridDim.x) {
     const int smp = idx ? idx[sidx] : sidx;
+    const bool first = sidx == int(blockIdx.x);
     __syncthreads();
     for (int i = threadIdx.x; i < PV; i += NT) S.x0[i] = in[size_t(smp) * PV + i];
-    zero_act(S.a1);
-    zero_act(S.a2);
-    zero_act(S.a3);
-    zero_act(S.d);
-    zero_act(S.e);
     __syncthreads();
     conv_in(S.x0, S.w0, S.a1);
     __syncthreads();
@@ -472,58 +566,49 @@ __global__ void __launch_bounds__(NT, 1) k_cnn_train(CnnWeights W, const float* 
     __syncthreads();
     if (!backward) continue;
     // ---- layer 3 (C -> 1): dW3[ci][tap] = sum_v a3[v+tap][ci] dz[v]
-    for (int i = threadIdx.x; i < CNN_W3; i += NT) {
-      const int ci = i / 27, tap = i % 27;
-      const int dx = tap % 3 - 1, dy = (tap / 3) % 3 - 1, dz = tap / 9 - 1;
-      float s = 0.f;
-      for (int c = 0; c < BN; ++c) {
-        const int x = (c & 7) + dx, y = ((c >> 3) & 7) + dy, z = (c >> 6) + dz;
-        s = fmaf(bf2f(S.a3.v[ci >> 3][pv(x, y, z)][ci & 7]), S.z[c], s);
-      }
-      gp[OFF_W3 + i] += s;
-    }
+    auto shifted = [](int tap, int c) {
+      return pv((c & 7) + tap % 3 - 1, ((c >> 3) & 7) + (tap / 3) % 3 - 1, (c >> 6) + tap / 9 - 1);
+    };
+    wgrad_1c(S.a3, [&](int, int c) { return S.z[c]; }, shifted, gp + OFF_W3, first);
     // da3[u][ci] = sum_tap W3[ci][tap] dz[u - (tap-1)] -> S.d (BF16)
     for (int c = threadIdx.x; c < BN; c += NT) {
       const int x = c & 7, y = (c >> 3) & 7, zz = c >> 6;
       float acc[CNN_C];
 #pragma unroll
       for (int ci = 0; ci < CNN_C; ++ci) acc[ci] = 0.f;
+#pragma unroll 1
       for (int tap = 0; tap < 27; ++tap) {
         const int X = x - (tap % 3 - 1), Y = y - ((tap / 3) % 3 - 1), Z = zz - (tap / 9 - 1);
         if (X < 0 || Y < 0 || Z < 0 || X > 7 || Y > 7 || Z > 7) continue;
         const float dzv = S.z[X + 8 * Y + 64 * Z];
+        float w[CNN_C];
+        tap_weights(S.w3, tap, w);
 #pragma unroll
-        for (int ci = 0; ci < CNN_C; ++ci) acc[ci] = fmaf(S.w3[ci * 27 + tap], dzv, acc[ci]);
+        for (int ci = 0; ci < CNN_C; ++ci) acc[ci] = fmaf(w[ci], dzv, acc[ci]);
       }
       const int p = pv(x, y, zz);
-#pragma unroll
-      for (int ci = 0; ci < CNN_C; ++ci) {
-        S.d.v[ci >> 3][p][ci & 7] = f2bf(acc[ci]);
-      }
+      pack8(&S.d.v[0][p][0], &acc[0]);
+      pack8(&S.d.v[1][p][0], &acc[8]);
     }
     __syncthreads();
     // ---- layer 2 (C -> C): weight gradient from a2 and dpre3 (S.d)
-    wgrad_cc(S.a2, S.d, gp + OFF_W2);
+    wgrad_cc(S.a2, S.d, gp + OFF_W2, first);
     __syncthreads();
     // da2 = W2^T (*) da3 -> S.e
     conv_cc(S.d, S.w2t, S.e);
     __syncthreads();
     // ---- layer 1 (C -> C)
-    wgrad_cc(S.a1, S.e, gp + OFF_W1);
+    wgrad_cc(S.a1, S.e, gp + OFF_W1, first);
     __syncthreads();
     conv_cc(S.e, S.w1t, S.d);  // da1 -> S.d
     __syncthreads();
     // ---- layer 0 (1 -> C): dW0[co][tap] = sum_v x0[v+tap] da1[v][co]
-    for (int i = threadIdx.x; i < CNN_W0; i += NT) {
-      const int co = i / 27, tap = i % 27;
-      const int dx = tap % 3, dy = (tap / 3) % 3, dz = tap / 9;
-      float s = 0.f;
-      for (int c = 0; c < BN; ++c) {
-        const int x = c & 7, y = (c >> 3) & 7, z = c >> 6;
-        s = fmaf(S.x0[(x + dx) + 10 * ((y + dy) + 10 * (z + dz))], bf2f(S.d.v[co >> 3][pv(x, y, z)][co & 7]), s);
-      }
-      gp[OFF_W0 + i] += s;
-    }
+    wgrad_1c(
+        S.d,
+        [&](int tap, int c) {
+          return S.x0[((c & 7) + tap % 3) + 10 * ((((c >> 3) & 7) + (tap / 3) % 3) + 10 * ((c >> 6) + tap / 9))];
+        },
+        [](int, int c) { return pv_of_cell(c); }, gp + OFF_W0, first);
   }
   // loss partial
   for (int o = 16; o > 0; o >>= 1) loss += __shfl_xor_sync(0xffffffffu, loss, o);
@@ -652,7 +737,6 @@ int cnn_train_step(const CnnWeights& W, float* adam_m, float* adam_v, int t, flo
   // the tensor-core layers read BF16 copies of the weights: refresh them from
   // the updated masters, so the next step's forward and backward use the
   // weights being trained
-  if (int rc = cnn_pack(W, s)) return rc;
   return cnn_pack(W, s);
 }
 
