@@ -386,8 +386,7 @@ int launch_pressure_rhs(const DevMesh& M, const double* vel, const double* pold,
 // ---------------------------------------------------------------------------
 // Mean removal + incremental pressure (PressureProjection.cpp:404-446) fused
 // with KernelGradP (:244-323) and the velocity update (:451-467).  The
-// pressure p = phi - avg (+ p_old) is formed at the point of use; the mean
-// drops out of the differences.
+// pressure p = phi - avg (+ p_old) is formed at the point of use.
 // ---------------------------------------------------------------------------
 template <int USE_POLD>
 __global__ void __launch_bounds__(PT, 6)
@@ -448,13 +447,14 @@ __global__ void __launch_bounds__(PT, 6)
     for (int d = 0; d < 2; ++d) {
       const Edge fm = edge_of(H, phi, gp, 2 * d, 1.0), fp = edge_of(H, phi, gp, 2 * d + 1, 1.0);
       double g[8];
-#pragma unroll
-      for (int z = 0; z < 8; ++z) g[z] = fp.at(z) - fm.at(z);
       if (USE_POLD) {
         // the scratch holds phi + p_old: nothing to add at its lanes
         const Edge om = edge_of(H, pold, nullptr, 2 * d, 1.0), op = edge_of(H, pold, nullptr, 2 * d + 1, 1.0);
 #pragma unroll
-        for (int z = 0; z < 8; ++z) g[z] += op.at(z) - om.at(z);
+        for (int z = 0; z < 8; ++z) g[z] = ((fp.at(z) - avg) + op.at(z)) - ((fm.at(z) - avg) + om.at(z));
+      } else {
+#pragma unroll
+        for (int z = 0; z < 8; ++z) g[z] = (fp.at(z) - avg) - (fm.at(z) - avg);
       }
 #pragma unroll
       for (int z = 0; z < 8; ++z) g[z] *= fac;
