@@ -11,7 +11,8 @@
 // columns, writes the result.
 //
 // What bounds it: WENO5 the FP64 pipe (about 213k FP64 instructions a thread
-// block, 27 us a stage on the 2340-block sphere mesh), upwind5 the L2 traffic
+// block, 27 us a stage on the 2340-block sphere mesh; a stage takes 89 us there
+// by events), upwind5 the L2 traffic
 // of the block and its ghosts (39 KB in, 24 KB out a block).  The layout
 // serves the sweeps: rows padded to 9 values and planes to 72, so that the
 // lines of a half-warp fall into different banks in x and y; ghost layers
@@ -49,22 +50,6 @@ struct AdvectSmem {
 };
 
 __device__ __forceinline__ double sq(double a) { return a * a; }
-
-// num / den for the reconstruction's denominators (1e-21 and up, far from the
-// ends of the exponent range): the hardware's reciprocal seed (rcp.approx,
-// about 20 bits), one third-order step r (1 + e + e^2) with e = 1 - den r
-// (Householder's iteration for 1/x), and the quotient corrected by its own
-// remainder.  Within 1 unit in the last place of the IEEE quotient; the
-// operator `/` costs four more FP64 instructions and a call for its special
-// cases, around which the sweep's registers would be saved.
-__device__ __forceinline__ double quotient(double num, double den) {
-  double r;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(den));
-  const double e = fma(-den, r, 1.0);
-  r = fma(r, fma(e, e, e), r);
-  const double q = num * r;
-  return fma(fma(-den, q, num), r, q);
-}
 
 // The lines of direction d: the offset of line (a, b) (tangential coordinates
 // in increasing dimension order) and the stride along it.
@@ -156,7 +141,7 @@ struct Weno {
     const double q23 = q2 * q3, w2 = 6.0 * q3, w3 = 3.0 * q2;
     const double num = fma(q1, fma(w3, g3, w2 * g2), q23 * g1);
     const double den = fma(q1, w2 + w3, q23);
-    return quotient(num, den);
+    return num / den;
   }
 };
 

@@ -6,8 +6,7 @@ block and of fewer blocks than the launch has CTAs.
 
 Tolerance: 1e-12 of max|u|, as the other operator tests; both sides are FP64
 and differ in summation order only (a stage is some 200 operations a cell, so
-rounding stays below 1e-13; the reconstruction's quotients are within one unit
-in the last place of the IEEE ones).
+rounding stays below 1e-13).
 """
 import numpy as np
 import pytest
