@@ -82,7 +82,8 @@ struct Field {
 // child at the cell, for a finer one), at face cell (a, bb): the lab rules of
 // lab.cuh.  par: the block's index parities.  Out of line, as fine_sums: the
 // coarse-fine faces' loads would take the registers of every block's path.
-__device__ __noinline__ double cf_ghost(Field F, int nb, int par, int kind, int f, int a, int bb) {
+template <class V>
+__device__ __noinline__ double cf_ghost(V F, int nb, int par, int kind, int f, int a, int bb) {
   const int d = f >> 1, s = f & 1;
   if (kind == K_FINER) {
     double sum = 0.0;
@@ -179,66 +180,123 @@ __device__ __forceinline__ double z_end(const Half& H, const double* v, const do
   return g ? g[32 * f + H.lane] : 0.0;
 }
 
-struct UdefGet {
-  ObstacleView ob;
-  const double* chi;
-  int c;
-  __device__ __forceinline__ double operator()(int blk, int cell) const {
-    const int sl = ob.slot[blk];
-    if (sl < 0) return 0.0;
-    return chi[size_t(blk) * BN + cell] <= ob.chi[size_t(sl) * BN + cell]
-               ? ob.udef[(size_t(c) * ob.nslots + sl) * BN + cell]
-               : 0.0;
+// u_def of one block, one component: the value of the body in slot sl where
+// the grid's chi is its own (sl < 0: the block holds none).
+struct Udef {
+  const double* u;
+  const double* body;
+  const double* grid;
+  __device__ __forceinline__ Udef(const ObstacleView& ob, const double* chi, int c, int blk, int sl)
+      : u(sl < 0 ? nullptr : ob.udef + (size_t(c) * ob.nslots + sl) * BN),
+        body(ob.chi + size_t(sl < 0 ? 0 : sl) * BN),
+        grid(chi + size_t(blk) * BN) {}
+  __device__ __forceinline__ double operator()(int, int cell) const {
+    const double g = grid[cell], o = body[cell], v = u[cell];  // together: v does not wait for the test
+    return g <= o ? v : 0.0;
+  }
+  __device__ __forceinline__ double at(int cell) const { return u ? (*this)(0, cell) : 0.0; }
+  // the column of eight cells from `cell` on
+  __device__ __forceinline__ void column(int cell, double (&v)[8]) const {
+#pragma unroll
+    for (int z = 0; z < 8; ++z) v[z] = 0.0;
+    if (u)
+#pragma unroll
+      for (int z = 0; z < 8; ++z) v[z] = (*this)(0, cell + z * 64);
   }
 };
 
-// Any neighbour value of u_def by the lab rules, one cell at a time (the rare
-// blocks next to a deforming body).
-__device__ __noinline__ double udef_at(const DevMesh& M, const UdefGet& get, int b, int x, int y, int z) {
-  const int q[3] = {x, y, z};
-  for (int d = 0; d < 3; ++d) {
-    if (q[d] >= 0 && q[d] < BS) continue;
-    const int s = q[d] < 0 ? 0 : 1, f = 2 * d + s, kind = M.fkind[6 * b + f];
-    const int* nb = M.fnbr + 24 * b + 4 * f;
-    const int a = q[tan1(d)], bb = q[tan2(d)];
-    if (kind == K_SAME) return get(nb[0], face_cell(d, 1 - s, 0, a, bb));
-    if (kind == K_BOUNDARY) {
-      const double v = get(b, face_cell(d, s, 0, a, bb));
-      return (nb[0] == BCK_WALL || get.c == d) ? -v : v;
+// The divergence of u_def (differences of the two neighbours, not scaled) on
+// the thread's column, to dv[8][32].  Component by component: a column comes
+// with eight independent loads a field, the x and y neighbours from the lanes
+// that hold them, and only the lanes at the half block's sides read on; gd: the
+// coarse-fine ghosts.  (A neighbour at a time, 48 dependent calls a thread,
+// the right-hand side next to a deforming body took 57 us on a box of 512
+// blocks and 300 us on a refined mesh of 2624 blocks, 1519 of them with body
+// cells; now 21 and 122, of which 12 and 64 without the deformation.)
+__device__ __forceinline__ void udef_divergence(const Half& H, const ObstacleView& ob, const double* chi,
+                                                const double* gd, double* dv) {
+  const int sl = ob.slot[H.b];
+#pragma unroll 1
+  for (int c = 0; c < 3; ++c) {
+    double d[8], t[8];
+    Udef(ob, chi, c, H.b, sl).column(H.cell0, d);
+#pragma unroll
+    for (int z = 0; z < 8; ++z) t[z] = c == 2 && z < 7 ? d[z + 1] : 0.0;
+#pragma unroll
+    for (int z = 1; z < 8; ++z) t[z] -= c == 2 ? d[z - 1] : 0.0;
+#pragma unroll 1
+    for (int s = 0; s < 2; ++s) {
+      const int f = 2 * c + s, kind = H.kind(f), n = H.nb(f);
+      const double sg = s ? 1.0 : -1.0;
+      if (c == 2) {
+        double e;
+        if (kind == K_SAME)
+          e = Udef(ob, chi, c, n, ob.slot[n]).at(H.cell0 + (s ? 0 : 7 * 64));
+        else if (kind == K_BOUNDARY)
+          e = s ? -d[7] : -d[0];
+        else
+          e = gd[32 * f + H.lane];
+        t[0] += s ? 0.0 : sg * e;
+        t[7] += s ? sg * e : 0.0;
+        continue;
+      }
+      const int step = c ? 8 : 1, row = H.lane >> 3;
+      double w[8];
+#pragma unroll
+      for (int z = 0; z < 8; ++z) w[z] = __shfl_sync(0xffffffffu, d[z], H.lane + (s ? step : -step));
+      const bool face = (c ? H.gy : H.gx) == (s ? BS - 1 : 0);  // at the block's face
+      if (face || (c && row == (s ? 3 : 0))) {
+        if (!face || kind == K_SAME) {
+          const int blk = face ? n : H.b;
+          Udef(ob, chi, c, blk, ob.slot[blk]).column(H.cell0 + (face ? (s ? -7 : 7) : (s ? 1 : -1)) * step, w);
+        } else {
+#pragma unroll
+          for (int z = 0; z < 8; ++z)
+            w[z] = kind == K_BOUNDARY ? -d[z] : gd[c ? 64 + H.gx + 8 * z : 32 * s + 8 * row + z];
+        }
+      }
+#pragma unroll
+      for (int z = 0; z < 8; ++z) t[z] += sg * w[z];
     }
-    if (kind == K_FINER) {
-      const int ch = nb[(a >> 2) + 2 * (bb >> 2)];
-      double sum = 0.0;
-      for (int e = 0; e < 8; ++e)
-        sum += get(ch, face_cell(d, 1 - s, e & 1, 2 * (a & 3) + ((e >> 1) & 1), 2 * (bb & 3) + (e >> 2)));
-      return 0.125 * sum;
-    }
-    const int h1 = M.index[3 * b + tan1(d)] & 1, h2 = M.index[3 * b + tan2(d)] & 1;
-    const int cb = nb[0];
-    return c2f_ghost([&](int cell) { return get(cb, cell); }, d, s, 1, a, bb, h1, h2);
+#pragma unroll
+    for (int z = 0; z < 8; ++z) dv[32 * z + H.lane] = c ? dv[32 * z + H.lane] + t[z] : t[z];
   }
-  return get(b, x + BS * y + BS * BS * z);
 }
 
 // The u_def part of the flux correction at face cell (a, bb) of finer face f
 // of a block next to a deforming body: chi times the face values, coarse and
-// fine (kernelUpdateTmpV with the flux correction).
-__device__ __noinline__ double udef_correction(const DevMesh& M, const UdefGet& get, const double* chi, int b, int f, int a, int bb,
-                                  double fac, double facf) {
-  const int d = f >> 1, s = f & 1;
+// fine (kernelUpdateTmpV with the flux correction).  ch: the child there, gd:
+// the block's ghost.  The four fine ghosts come from this block's cells and
+// share their nodes (child_ghost1).
+__device__ __noinline__ double udef_correction(ObstacleView ob, const double* chi, int b, int ch, int f, int a, int bb,
+                                               double gd, double fac, double facf) {
+  const int d = f >> 1, s = f & 1, oc = face_cell(d, s, 0, a, bb);
   const double sg = s ? -1.0 : 1.0;
-  const int oc = face_cell(d, s, 0, a, bb);
-  int q[3];
-  q[d] = s ? BS : -1;
-  q[tan1(d)] = a;
-  q[tan2(d)] = bb;
-  double v = -sg * chi[size_t(b) * BN + oc] * fac * (udef_at(M, get, b, q[0], q[1], q[2]) + get(b, oc));
-  const int ch = M.fnbr[24 * b + 4 * f + (a >> 2) + 2 * (bb >> 2)];
+  const Udef own(ob, chi, d, b, ob.slot[b]), fine(ob, chi, d, ch, ob.slot[ch]);
+  double v = -sg * chi[size_t(b) * BN + oc] * fac * (gd + own.at(oc));
+  int n1, n2;
+  double wn[3], w1[2][3], w2[2][3], g[4] = {0.0, 0.0, 0.0, 0.0};
+  lagrange3(-0.25, wn);
+#pragma unroll
+  for (int e = 0; e < 2; ++e) {
+    tan_stencil(2 * (a & 3) + e, a >> 2, n1, w1[e]);
+    tan_stencil(2 * (bb & 3) + e, bb >> 2, n2, w2[e]);
+  }
+  if (own.u)
+#pragma unroll
+    for (int j = 0; j < 3; ++j)
+#pragma unroll
+      for (int i = 0; i < 3; ++i) {
+        double q = 0.0;
+#pragma unroll
+        for (int k = 0; k < 3; ++k) q = fma(wn[k], own(b, face_cell(d, s, k, n1 + i, n2 + j)), q);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) g[e] = fma(w2[e >> 1][j] * w1[e & 1][i], q, g[e]);
+      }
+#pragma unroll
   for (int e = 0; e < 4; ++e) {
-    const int fa = 2 * (a & 3) + (e & 1), fb = 2 * (bb & 3) + (e >> 1);
-    const int cf = face_cell(d, 1 - s, 0, fa, fb);
-    const double gd = child_ghost1([&](int cell) { return get(b, cell); }, M, ch, d, s, fa, fb);
-    v += sg * chi[size_t(ch) * BN + cf] * facf * (gd + get(ch, cf));
+    const int cf = face_cell(d, 1 - s, 0, 2 * (a & 3) + (e & 1), 2 * (bb & 3) + (e >> 1));
+    v += sg * chi[size_t(ch) * BN + cf] * facf * (g[e] + fine.at(cf));
   }
   return v;
 }
@@ -255,11 +313,14 @@ __global__ void __launch_bounds__(PT, 6)
     k_pressure_rhs(DevMesh M, const double* __restrict__ vel, const double* __restrict__ pold,
                    const double* __restrict__ chi, ObstacleView ob, double dt, double* __restrict__ lhs,
                    double* __restrict__ phi) {
-  __shared__ double scratch[PT / 32][3 * kGhosts];
+  // near a deforming body also u_def's ghosts and its divergence
+  __shared__ double scratch[PT / 32][3 * kGhosts + (NEAR ? kGhosts + 8 * 32 : 0)];
   const int warp = threadIdx.x >> 5;
   double* gu = scratch[warp];
   double* gp = gu + kGhosts;
   double* corr = gp + kGhosts;
+  double* gd = corr + kGhosts;
+  double* dv = gd + kGhosts;
   const size_t n = size_t(M.nb) * BN;
   Half H;
   for (int b = blockIdx.x * PBLOCKS + (warp >> 1); b < M.nb; b += gridDim.x * PBLOCKS) {
@@ -269,9 +330,9 @@ __global__ void __launch_bounds__(PT, 6)
     const bool near = NEAR && ob.near[b] != 0;
     auto U = [&](int d) { return Field{vel + d * n, nullptr, 0.0}; };
     const Field P{pold, nullptr, 0.0};
-    // the correction of the right-hand side at a finer face's cell; gn, gq:
-    // the ghosts there
-    auto correction = [&](int f, int a, int bb, double gn, double gq) {
+    // the correction of the right-hand side at a finer face's cell; gn, gq,
+    // gs: the ghosts there of the velocity, p_old and u_def
+    auto correction = [&](int f, int a, int bb, double gn, double gq, double gs) {
       const int d = f >> 1, s = f & 1, oc = face_cell(d, s, 0, a, bb), ch = H.nb_at(f, a, bb);
       const double hf = 0.5 * h, facf = 0.25 * fac;  // h = h0 2^-level: exact
       const double sg = s ? -1.0 : 1.0;
@@ -281,7 +342,7 @@ __global__ void __launch_bounds__(PT, 6)
         const double2 p = fine_sums(P, b, ch, f, a, bb);
         v -= h * (pold[H.own + oc] - gq) + hf * (p.x - p.y);
       }
-      if (near) v += udef_correction(M, UdefGet{ob, chi, d}, chi, b, f, a, bb, fac, facf);
+      if (near) v += udef_correction(ob, chi, b, ch, f, a, bb, gs, fac, facf);
       return v;
     };
     __syncwarp();  // the last block's lanes are done with the scratch
@@ -289,11 +350,18 @@ __global__ void __launch_bounds__(PT, 6)
       const int nb = H.nb_at(f, a, bb);
       const double u = cf_ghost(U(f >> 1), nb, H.par, kind, f, a, bb);
       const double p = USE_POLD ? cf_ghost(P, nb, H.par, kind, f, a, bb) : 0.0;
+      double ud = 0.0;
+      if (near) {
+        const int sl = ob.slot[nb];
+        if (sl >= 0) ud = cf_ghost(Udef(ob, chi, f >> 1, nb, sl), nb, H.par, kind, f, a, bb);
+        gd[i] = ud;
+      }
       gu[i] = u;
       if (USE_POLD) gp[i] = p;
-      if (kind == K_FINER) corr[i] = correction(f, a, bb, u, p);
+      if (kind == K_FINER) corr[i] = correction(f, a, bb, u, p, ud);
     });
     __syncwarp();
+    if (near) udef_divergence(H, ob, chi, gd, dv);
     const int fy = 2 + H.half;
     const double* w = vel + 2 * n + H.own + H.cell0;
     const Edge um = edge_of(H, vel, gu, 0, -1.0), up = edge_of(H, vel, gu, 1, -1.0);
@@ -307,22 +375,9 @@ __global__ void __launch_bounds__(PT, 6)
       const double lo = z > 0 ? wc[z - 1] : wm, hi = z < 7 ? wc[z + 1] : wp;
       out[z] = fac * (up.at(z) - um.at(z) + vp.at(z) - vm.at(z) + hi - lo);
     }
-    if (near) {
-#pragma unroll 1
-      for (int z = 0; z < 8; ++z) {
-        double div = 0.0;
-#pragma unroll 1
-        for (int c = 0; c < 3; ++c) {
-          const UdefGet D{ob, chi, c};
-          const int x = H.gx, y = H.gy;
-          div += udef_at(M, D, b, x + (c == 0), y + (c == 1), z + (c == 2)) -
-                 udef_at(M, D, b, x - (c == 0), y - (c == 1), z - (c == 2));
-        }
-        const double v = -chi[H.own + H.cell0 + z * 64] * fac * div;
+    if (near)
 #pragma unroll
-        for (int k = 0; k < 8; ++k) out[k] += k == z ? v : 0.0;
-      }
-    }
+      for (int z = 0; z < 8; ++z) out[z] += -chi[H.own + H.cell0 + z * 64] * fac * dv[32 * z + H.lane];
     if (USE_POLD) {
       double pc[8];
 #pragma unroll
