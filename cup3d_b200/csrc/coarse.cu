@@ -469,16 +469,18 @@ __global__ void __launch_bounds__(NT) k_coarse_mean(int nb, const double* __rest
 // end of the pivot order, checked by A^-1 (A v) = v to 1e-6 for the probe
 // vector v; when a pivot block has a small pivot or the check fails, the
 // inverse is redone by column-wise Gauss-Jordan with partial pivoting
-// (*fallback = 1).  Returns CUP_ERR_MESH for a singular matrix.
+// (*fallback = 1).  Returns CUP_ERR_MESH for a singular matrix.  scratch: kept
+// by the caller (null: freed on return), allocated with room for `room` unknowns
+// when it is too small.
 int device_inverse_dev(double* M, int n, int last, int sms, cudaStream_t s, int* fallback,
-                       InverseScratch* scratch) {
+                       InverseScratch* scratch, int room) {
   if (fallback) *fallback = 0;
   InverseScratch local;
   InverseScratch& X = scratch ? *scratch : local;
   if (X.cap < n) {
     X.arena.release();
     X.cap = 0;
-    const size_t cap = scratch ? size_t(n) + n / 4 : size_t(n);
+    const size_t cap = std::max(n, room);
     // one allocation, carved up: the first call pays for each
     double* base = nullptr;
     if (int rc = X.arena.alloc(&base, cap * cap + GJB * GJB + 2 * size_t(GJB) * cap + 3 * cap + 1)) return rc;
@@ -669,7 +671,7 @@ int coarse_build(cup_ctx* c) {
   // thousand blocks)
   {
     int fb = 0;
-    if (int rc = device_inverse_dev(Ac, nb, mode == 1 ? mb : -1, c->num_sms, s, &fb, &C.iscratch))
+    if (int rc = device_inverse_dev(Ac, nb, mode == 1 ? mb : -1, c->num_sms, s, &fb, &C.iscratch, nb + nb / 4))
       return rc == CUP_ERR_MESH ? set_error(CUP_ERR_MESH, "two-level preconditioner: singular coarse operator") : rc;
     C.pivoted = fb;
     k_to_float<<<std::max(1, std::min(nb, c->num_sms * 8)), NT, 0, s>>>(Ac, nb, C.inv);
@@ -717,14 +719,20 @@ int cup_coarse_matrix(cup_ctx* c, double* out, int32_t* colours) {
   return 0;
 }
 
+// Direct calls use the coarse set-up's scratch and leave it with the context up
+// to this size (35 MB), in exactly the room they need; beyond it the scratch is
+// the call's own, so that a large inverse holds no memory afterwards.
+// Allocating and freeing it costs 0.7 to 0.9 ms a call: of 1.9 ms at 604
+// unknowns, of 5.6 at 2049, of 10.1 at 3000.
+constexpr int kInverseKeep = 2048;
+
 int cup_dense_inverse_dev(cup_ctx* c, double* d_a, int32_t n, int32_t last, int32_t* pivoted) {
   ProfBind pb_(c);
   if (!c || !d_a || n <= 0 || last < -1 || last >= n || c->host_only)
     return ctx_fail(c, CUP_ERR_ARG, "cup_dense_inverse_dev: bad arguments");
   int fb = 0;
-  // the coarse set-up's scratch, kept with the context: allocating and freeing
-  // it took as long as the inverse of 604 unknowns (0.9 of 1.9 ms a call)
-  if (int rc = device_inverse_dev(d_a, n, last, c->num_sms, c->stream, &fb, &c->coarse.iscratch))
+  InverseScratch* kept = n <= kInverseKeep || n <= c->coarse.iscratch.cap ? &c->coarse.iscratch : nullptr;
+  if (int rc = device_inverse_dev(d_a, n, last, c->num_sms, c->stream, &fb, kept, n))
     return ctx_fail(c, rc, cup_last_error(nullptr));
   if (pivoted) *pivoted = fb;
   return 0;

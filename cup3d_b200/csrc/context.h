@@ -320,9 +320,10 @@ int coarse_build(cup_ctx* c);
 int device_inverse(const double* a, int n, double* d_inv, int sms, cudaStream_t s);
 // The inverse in place of an n x n device matrix, index `last` (>= 0) last in
 // the pivot order; *fallback = 1 when the pivoted column-wise form ran.
-// Scratch from `scratch` when given (kept for the next call), else allocated for the call.
+// Scratch from `scratch` when given (kept for the next call; allocated with room
+// for `room` unknowns when it is too small), else allocated for the call.
 int device_inverse_dev(double* M, int n, int last, int sms, cudaStream_t s, int* fallback,
-                       InverseScratch* scratch = nullptr);
+                       InverseScratch* scratch = nullptr, int room = 0);
 // The learned map of the current weights for the solver (folds them when they
 // changed; the lab buffer for the current mesh).
 int lmap_prepare(cup_ctx* c, LocalMap* out);

@@ -430,7 +430,9 @@ int cup_cnn_forward_host_noalloc(cup_ctx* ctx, const float* in, float* out, int3
  * the end of the pivot order, checked by A^-1 (A v) = v to 1e-6 for a fixed
  * probe v; when a pivot block is near-singular or the check fails, column-wise
  * Gauss-Jordan with partial pivoting, and *pivoted (may be NULL) = 1.
- * CUP_ERR_MESH for a singular matrix. */
+ * CUP_ERR_MESH for a singular matrix.  Scratch: n^2 + 67 n + 1025 doubles; up to
+ * n = 2048 (35 MB) the context keeps it until it is closed, beyond that it is
+ * freed on return. */
 int cup_coarse_matrix(cup_ctx* ctx, double* out, int32_t* colours);
 int cup_coarse_apply_dev(cup_ctx* ctx, const double* d_r, double* d_z);
 int cup_dense_inverse_dev(cup_ctx* ctx, double* d_a, int32_t n, int32_t last, int32_t* pivoted);

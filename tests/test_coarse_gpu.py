@@ -192,3 +192,20 @@ def test_dense_inverse_singular_matrix_is_an_error():
     a = torch.tensor(A, device="cuda")
     assert not ctx.dense_inverse(a)
     assert np.abs(a.cpu().numpy() - np.eye(40) / 3.0).max() <= 1e-15
+
+
+@pytest.mark.parametrize("n,kept", [(2048, 1.1), (3000, 0.0)])
+def test_dense_inverse_scratch_is_bounded(n, kept):
+    # the context keeps the scratch (n^2 doubles and a little) of calls of up
+    # to 2048 unknowns, in the room that they need, and none of larger ones
+    import torch
+    ctx = make_ctx("amr2_free", device=0)
+    for _ in range(2):  # the kernels are loaded
+        ctx.dense_inverse(torch.eye(64, dtype=torch.float64, device="cuda"))
+    a = 3.0 * torch.eye(n, dtype=torch.float64, device="cuda")
+    torch.cuda.synchronize()
+    before = torch.cuda.mem_get_info()[0]
+    assert not ctx.dense_inverse(a)
+    held = before - torch.cuda.mem_get_info()[0]
+    assert held <= kept * 8 * n * n + (4 << 20), held  # 4 MB: the allocator's granularity
+    assert float((a - torch.eye(n, dtype=torch.float64, device="cuda") / 3.0).abs().max()) <= 1e-15
