@@ -1224,7 +1224,8 @@ __device__ __forceinline__ void p3_block(const KArgs<T>& A, const GroupIdx& G, G
 constexpr size_t kSmemCache = BN * sizeof(double);
 constexpr size_t kSmemTiles = kSmemCache + PGROUPS * KB_CACHE * sizeof(BlockInfo);
 constexpr size_t kPersistentSmem = kSmemTiles + PGROUPS * sizeof(GroupTile);
-// columns of the restriction that the coarse phase stages at once, over the tiles
+// columns of the restriction that fit over the tiles: the coarse phase stages
+// it whole up to this many blocks and reads it from global memory beyond
 constexpr int kStageCols = int(PGROUPS * sizeof(GroupTile) / sizeof(double)) & ~63;
 constexpr size_t kLearnedSmem = std::max(kPersistentSmem, kSmemTiles + LMAP_TILE_BYTES);
 static_assert(kSmemTiles % 16 == 0, "tiles and staged labs start 16-byte aligned");

@@ -95,3 +95,26 @@ def test_batched_twolevel_mixed_precision():
         x64, x32 = sols["b200_twolevel"][0][k], sols["b200_twolevel_mixed"][0][k]
         assert np.linalg.norm(x32 - x64) <= 1e-8 * np.linalg.norm(x64), k
     assert sum(sols["b200_twolevel_mixed"][1]) < sum(sols["b200_mixed"][1]), sols
+
+
+def test_batched_twolevel_past_the_staged_restriction():
+    # A group stages its case's restriction up to 1203 blocks and reads it from
+    # global memory beyond: a case on either side of the limit against the same
+    # case alone.
+    from cup3d_b200.workloads import make_swarm_ctx, swarm_rhs
+    which = (0, 4)
+    ctxs = [make_swarm_ctx(i, 0, "-poissonSolver b200_twolevel -poissonTol 0 -poissonTolRel 1e-8") for i in which]
+    assert ctxs[0].nb <= 1203 < ctxs[1].nb
+    batch = cup.Batch(ctxs)
+    bs = [swarm_rhs(c, i) for c, i in zip(ctxs, which)]
+    xd = torch_dev(np.zeros(sum(len(b) for b in bs)))
+    rc, stats = batch.poisson_solve_dev(torch_dev(np.concatenate(bs)), xd)
+    assert rc == 0
+    for ctx, b, x, st in zip(ctxs, bs, split(batch, xd.cpu().numpy()), stats):
+        xa = torch_dev(np.zeros(len(b)))
+        rca, sta = ctx.poisson_solve_dev(torch_dev(b), xa)
+        assert rca == 0 and sta["status"] == 1 and st["status"] == 1
+        xa = xa.cpu().numpy()
+        print(ctx.nb, "blocks, iterations: batched", st["iterations"], "alone", sta["iterations"])
+        assert np.linalg.norm(x - xa) <= 1e-6 * np.linalg.norm(xa)
+        assert abs(st["iterations"] - sta["iterations"]) <= max(2, sta["iterations"] // 10)

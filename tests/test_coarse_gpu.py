@@ -194,6 +194,30 @@ def test_dense_inverse_singular_matrix_is_an_error():
     assert np.abs(a.cpu().numpy() - np.eye(40) / 3.0).max() <= 1e-15
 
 
+def test_twolevel_past_the_staged_restriction():
+    # The persistent solver stages the restriction in shared memory up to 4800
+    # blocks and reads it from global memory beyond; the host-driven form
+    # multiplies by A_c^-1 in a kernel of its own.  The same method, summed in
+    # other orders: the counts and solutions of the two agree as they do below
+    # the limit.
+    from cup3d_b200.workloads import make_sphere_re1000_ctx
+    sols = {}
+    for pers in (1, 0):
+        ctx = make_sphere_re1000_ctx(0, f"b200 -poissonPersistent {pers}")
+        assert ctx.nb > 4800
+        hh = np.repeat(ctx.blocks()[2], 512)
+        b = np.random.default_rng(11).standard_normal(len(hh))
+        b -= np.sum(b * hh ** 3) / np.sum(hh ** 3)
+        bd, xd = torch_dev(b), torch_dev(np.zeros(len(b)))
+        ctx.set_poisson("b200_twolevel", 0.0, 1e-8, 1000)
+        rc, st = ctx.poisson_solve_dev(bd, xd)
+        assert rc == 0 and st["status"] == 1 and st["true_rel"] <= 1.5e-8, (pers, st)
+        sols[pers] = (xd.cpu().numpy(), st["iterations"])
+    print("iterations persistent / host-driven:", sols[1][1], sols[0][1])
+    assert abs(sols[1][1] - sols[0][1]) <= max(2, sols[1][1] // 10)
+    assert np.linalg.norm(sols[1][0] - sols[0][0]) <= 1e-6 * np.linalg.norm(sols[1][0])
+
+
 @pytest.mark.parametrize("n,kept", [(2048, 1.1), (3000, 0.0)])
 def test_dense_inverse_scratch_is_bounded(n, kept):
     # the context keeps the scratch (n^2 doubles and a little) of calls of up
