@@ -22,7 +22,7 @@
 // let four CTAs stay on an SM, whose copies and sweeps overlap.
 #include "../../include/cup3d_b200.h"
 #include "profiler.h"
-#include "staged.cuh"
+#include "block_meta.cuh"
 #include "stencils.cuh"
 
 namespace cup3d {

@@ -122,7 +122,7 @@ static int batch_coarse_setup(cup_ctx* c, cup_ctx* const* cases) {
   for (int k = 0; k < c->ncase; ++k) {
     const long long n = c->case_first[k + 1] - c->case_first[k];
     off[k] = total;
-    total += n * coarse_ld(int(n));
+    total += n * n;
   }
   DevArena& A = c->bcoarse_arena;
   float* inv = nullptr;
@@ -145,8 +145,8 @@ static int batch_coarse_setup(cup_ctx* c, cup_ctx* const* cases) {
     if (int rc_ = coarse_build(s)) return rc_;
     const long long n = c->case_first[k + 1] - c->case_first[k];
     if (s->coarse.nb != n) return set_error(CUP_ERR_STATE, "batch two-level: a case's coarse space does not match");
-    CUP_CUDA_TRY(cudaMemcpyAsync(inv + off[k], s->coarse.inv, size_t(n * coarse_ld(int(n))) * sizeof(float),
-                                 cudaMemcpyDeviceToDevice, s->stream));
+    CUP_CUDA_TRY(cudaMemcpyAsync(inv + off[k], s->coarse.inv, size_t(n * n) * sizeof(float), cudaMemcpyDeviceToDevice,
+                                 s->stream));
     CUP_CUDA_TRY(cudaStreamSynchronize(s->stream));
   }
   c->bcoarse = BatchCoarse{inv, d_off, rc, rc2, yc, yc2, w};

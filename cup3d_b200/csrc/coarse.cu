@@ -421,21 +421,19 @@ __global__ void __launch_bounds__(NT) k_probe_check(const double* __restrict__ v
   }
 }
 
-// FP32 copy of an n x n device matrix, rows of coarse_ld(n) filled with zeros
-__global__ void k_to_float(const double* __restrict__ a, int n, float* __restrict__ out) {
-  const int ld = coarse_ld(n);
-  for (int i = blockIdx.x; i < n; i += gridDim.x)
-    for (int j = threadIdx.x; j < ld; j += blockDim.x)
-      out[size_t(i) * ld + j] = j < n ? float(a[size_t(i) * n + j]) : 0.f;
+// FP32 copy of a device array
+__global__ void k_to_float(const double* __restrict__ a, size_t n, float* __restrict__ out) {
+  for (size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += size_t(gridDim.x) * blockDim.x)
+    out[i] = float(a[i]);
 }
 
-// y = Ainv x (n rows of coarse_ld(n)): one warp per row
+// y = Ainv x (n x n, row-major): one warp per row
 __global__ void __launch_bounds__(NT) k_coarse_gemv(const float* __restrict__ Ainv, const double* __restrict__ x,
                                                     int n, double* __restrict__ y) {
   const int lane = threadIdx.x & 31;
   const int warps = blockDim.x >> 5;
   for (int row = blockIdx.x * warps + (threadIdx.x >> 5); row < n; row += gridDim.x * warps) {
-    const float* a = Ainv + size_t(row) * coarse_ld(n);
+    const float* a = Ainv + size_t(row) * n;
     double s = 0.0;
     for (int j = lane; j < n; j += 32) s += double(a[j]) * __ldg(x + j);
 #pragma unroll
@@ -622,7 +620,7 @@ int coarse_build(cup_ctx* c) {
     if (int rc = A.alloc(&C.yc, cap)) return rc;
     if (int rc = A.alloc(&C.rc2, cap)) return rc;
     if (int rc = A.alloc(&C.yc2, cap)) return rc;
-    if (int rc = A.alloc(&C.inv, cap * coarse_ld(int(cap)))) return rc;
+    if (int rc = A.alloc(&C.inv, cap * cap)) return rc;
     if (int rc = A.alloc(&C.ac, cap * cap)) return rc;
     if (int rc = A.alloc(&C.colour, cap)) return rc;
     if (int rc = A.alloc(&C.sum, cap)) return rc;
@@ -674,7 +672,7 @@ int coarse_build(cup_ctx* c) {
     if (int rc = device_inverse_dev(Ac, nb, mode == 1 ? mb : -1, c->num_sms, s, &fb, &C.iscratch, nb + nb / 4))
       return rc == CUP_ERR_MESH ? set_error(CUP_ERR_MESH, "two-level preconditioner: singular coarse operator") : rc;
     C.pivoted = fb;
-    k_to_float<<<std::max(1, std::min(nb, c->num_sms * 8)), NT, 0, s>>>(Ac, nb, C.inv);
+    k_to_float<<<std::max(1, c->num_sms * 8), NT, 0, s>>>(Ac, nn, C.inv);
     CUP_CUDA_TRY(cudaGetLastError());
     CUP_CUDA_TRY(cudaStreamSynchronize(s));
   }

@@ -454,7 +454,7 @@ struct KArgs {
   // two-level preconditioner (persistent solver): A_c^-1 (cnb x cnb, cnb = 0:
   // none), the restricted vectors of zv and zr and the blocks' 512 h^3
   int cnb;           // single case: blocks of A_c; batch: 1 when the cases carry coarse spaces
-  const long long* coff;  // batch: offset of each case's A_c^-1 (nb_c rows of coarse_ld(nb_c)) in cinv; null: one case
+  const long long* coff;  // batch: offset of each case's A_c^-1 (nb_c x nb_c) in cinv; null: one case
   const float* cinv;
   double* crc_v;
   double* crc_r;
@@ -1037,13 +1037,12 @@ template <class T, class Block>
 __device__ __forceinline__ double coarse_blocks(const KArgs<T>& A, const GroupIdx& G, int nblk, Block block,
                                                 const double* rc, int cf, int n, const float* inv, double* yc, T* v,
                                                 double* gsm) {
-  const int ld = coarse_ld(n);
   double added = 0.0;
 #pragma unroll 1
   for (int k = 0; k < nblk; k += 2) {
     const int b0 = block(k), b1 = block(min(k + 1, nblk - 1));
     double s[2] = {0.0, 0.0};
-    coarse_rows(inv + size_t(b0 - cf) * ld, inv + size_t(b1 - cf) * ld, rc, n, G.lane, s);
+    coarse_rows(inv + size_t(b0 - cf) * n, inv + size_t(b1 - cf) * n, rc, n, G.lane, s);
     group_reduce<2>(s, gsm, G);
 #pragma unroll
     for (int i = 0; i < 2; ++i) {

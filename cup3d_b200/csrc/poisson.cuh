@@ -74,7 +74,7 @@ struct BatchWork {
 };
 
 // The cases' two-level preconditioners in a batch: each case's A_c^-1
-// (nb_c rows of coarse_ld(nb_c), FP32) packed in case order (case c at off[c]),
+// (nb_c x nb_c, FP32, row-major) packed in case order (case c at off[c]),
 // the restriction buffers and 512 h^3 over the batch's blocks.
 struct BatchCoarse {
   const float* inv = nullptr;
@@ -85,9 +85,6 @@ struct BatchCoarse {
   double* yc2 = nullptr;
   const double* w = nullptr;
 };
-
-// Row length of A_c^-1 as stored: rows start on 16-byte boundaries.
-__host__ __device__ constexpr int coarse_ld(int n) { return (n + 3) & ~3; }
 
 struct SolveParams {
   double tol_abs, tol_rel;
@@ -112,7 +109,7 @@ int launch_block_inverse(const DevMesh& M, const double* in, double* out, Poisso
                          cudaStream_t s);
 // Solves A x = b; x holds the initial guess on entry and x_opt on exit.
 // Coarse space of the two-level preconditioners (built by coarse_build):
-// A_c^-1 (nb rows of coarse_ld(nb)), two restriction buffers, two buffers of
+// A_c^-1 (nb x nb, row-major), two restriction buffers, two buffers of
 // corrections and the blocks' 512 h^3.  nb = 0: no coarse correction.
 struct CoarseView {
   int nb;
