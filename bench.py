@@ -62,7 +62,7 @@ from cup3d_b200.workloads import (SPHERE_BODY, SPHERE_FLAGS, SPHERE_MESH, SPHERE
 ALG_BYTES = {
     "advect_stage_weno5": 8 * 10,       # mean over stages of 9S/12S/9S (R u, tmpV; W u, tmpV)
     "advect_stage_upwind5": 8 * 10,
-    "pressure_rhs": 8 * 7,              # R u(3), chi, p_old; W lhs, phi
+    "pressure_rhs": 8 * 6,              # R u(3), p_old; W lhs, phi (the bodies here are rigid: no u_def)
     "grad_update": 8 * 9,               # R phi, p_old, u(3); W u(3), p_new
     "bicg_a_pupdate_precond": 8 * 5,    # R r, p, nu; W p, z1
     "bicg_b_spmv_dot": 8 * 3,           # R z1, rhat; W nu
@@ -77,13 +77,13 @@ ALG_BYTES = {
 
 
 # DRAM bytes (read + write) per cell and iteration of the persistent solver,
-# measured by ncu (--set full) on 16 iterations of one solve on the sphere
-# mesh (1,198,080 cells), per solver:
-#   b200 (`python -m cup3d_b200.kernel_cases solve`): 147.7 MB + 594.2 MB,
+# measured by ncu on 16 iterations of one solve on the sphere mesh (1,198,080
+# cells), per solver:
+#   b200 (`python -m cup3d_b200.kernel_cases solve`): 263.2 MB + 716.8 MB,
 #     most of the 176 algorithmic bytes hit in L2;
-#   b200_twolevel (`... solve b200_twolevel`): 724.2 MB + 844.7 MB, the two
+#   b200_twolevel (`... solve b200_twolevel`): 832.3 MB + 829.1 MB, the two
 #     reads of the 21.9 MB A_c^-1 an iteration most of the growth.
-MEASURED_TRAFFIC_PER_CELL_ITER = {("bicg_persistent", "b200"): 38.70, ("bicg_persistent", "b200_twolevel"): 81.8}
+MEASURED_TRAFFIC_PER_CELL_ITER = {("bicg_persistent", "b200"): 51.1, ("bicg_persistent", "b200_twolevel"): 86.7}
 
 
 def dist_env():
@@ -552,10 +552,12 @@ def run_b200(args):
     per_launch_ms = dom_ms / max(dom_n, 1)
     if dom_name == "bicg_persistent":
         # one launch per solve, 176 B/cell per iteration; the two-level solver
-        # adds two coarse corrections per iteration: a read-modify-write of z
-        # (16 B/cell) and a row of A_c^-1 per block (8 nb^2 bytes) each
-        per_cell = ALG_BYTES[dom_name] + (32 if args.solver == "b200_twolevel" else 0)
-        per_iter = per_cell * ncell + (16 * nb * nb if args.solver == "b200_twolevel" else 0)
+        # adds two coarse corrections per iteration: A_c^-1 read whole (4 nb^2
+        # bytes, FP32) and a block's restriction and correction written and
+        # read (32 bytes) each
+        per_iter = ALG_BYTES[dom_name] * ncell
+        if args.solver == "b200_twolevel":
+            per_iter += 8 * nb * nb + 64 * nb
         alg_bytes = int(per_iter * sum(prof_iters) / max(dom_n, 1))
     else:
         alg_bytes = ALG_BYTES.get(dom_name, 0) * ncell
