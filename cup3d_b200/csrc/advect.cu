@@ -10,16 +10,15 @@
 // accumulator in shared memory; the z sweep, whose lines are coalesced
 // columns, writes the result.
 //
-// What bounds it: WENO5 the FP64 pipe (about 213k FP64 instructions a thread
-// block, 27 us a stage on the 2340-block sphere mesh; a stage takes 89 us there
-// by events), upwind5 the L2 traffic
-// of the block and its ghosts (39 KB in, 24 KB out a block).  The layout
-// serves the sweeps: rows padded to 9 values and planes to 72, so that the
-// lines of a half-warp fall into different banks in x and y; ghost layers
-// apart, [face][layer][line], read by the line's own index in all three
-// directions, so that one rolled loop runs them all (three unrolled copies
-// overflow the instruction cache).  55 KB of shared memory and 80 registers
-// let four CTAs stay on an SM, whose copies and sweeps overlap.
+// What bounds it: WENO5 the FP64 pipe and issue slots (43% and 58% busy; 90 us a
+// stage on the 2340-block sphere mesh), upwind5 the L2 traffic of the block and
+// its ghosts (39 KB in, 24 KB out a block).  The layout serves the sweeps: rows
+// padded to 9 values and planes to 72, so that the lines of a half-warp fall
+// into different banks in x and y; ghost layers apart, [face][layer][line],
+// read by the line's own index in all three directions, so that one rolled loop
+// runs them all (three unrolled copies overflow the instruction cache).  55 KB
+// of shared memory and 80 registers let four CTAs stay on an SM, whose copies
+// and sweeps overlap.
 #include "../../include/cup3d_b200.h"
 #include "profiler.h"
 #include "block_meta.cuh"

@@ -1,7 +1,7 @@
 // The projection's two stencil passes on the device (FP64): the Poisson
 // right-hand side and the gradient update.
 //
-// Both are bound by memory latency: 56 and 72 bytes a cell and a few dozen
+// Both are bound by memory latency: 48 and 72 bytes a cell and a few dozen
 // operations.  A warp takes half a block, four rows of eight z-columns; a
 // thread keeps its column in registers and reads the x and y neighbours by
 // plain loads, which hit L1 (the half block's own rows, or a neighbour's face

@@ -71,7 +71,7 @@ def test_projection_passes_match_oracle(name, step, body):
 @pytest.mark.parametrize("step", [1, 5])
 def test_deforming_body_next_to_a_rigid_one(step):
     # Every block next to a deforming body reads its u_def, chi and body chi
-    # beside the velocity (120 bytes a cell for 56): a right-hand side over
+    # beside the velocity (88 bytes a cell for 48): a right-hand side over
     # such blocks alone stays below 2.5 of the rigid body's time (1.5 and 1.7
     # measured; 3.9 when each neighbour is read by a call of its own).
     cfg = cup.config("-bpdx 8 -bpdy 8 -bpdz 8 -levelMax 1 -extent 1", device=0)
