@@ -69,7 +69,7 @@ def test_projection_passes_match_oracle(name, step, body):
 
 
 @pytest.mark.parametrize("step", [1, 5])
-def test_deforming_body_next_to_a_rigid_one(step):
+def test_deforming_body_time_against_a_rigid_one(step):
     # Every block next to a deforming body reads its u_def, chi and body chi
     # beside the velocity (88 bytes a cell for 48): a right-hand side over
     # such blocks alone stays below 2.5 of the rigid body's time (1.5 and 1.7
